@@ -36,11 +36,31 @@ namespace {
 
 const int kMaxDev = 64;
 
+/* launch mode until set_launch or GCCHEM_B200_MODE names a kernel: chosen per
+   call by the number of cells (auto_mode) */
+const int kAuto = -1;
+/* The cooperative kernel solves a cell in a thirtieth of the time one thread
+   takes, but keeps only a few cells per SM; one thread per cell catches up
+   once the batch fills the GPU.  Full cold steps on a B200, cooperative /
+   persistent: fullchem 1,000 cells 0.069 / 0.549 s, 16,000 cells 0.778 /
+   1.052 s, about even at 24,000.  Without the fused factorisation (synthetic
+   mechanism) the cooperative kernel wins at every size: 1,500 cells 0.050 /
+   0.692 s, 1.01 M / 0.82 M attempts per second at full load.  The
+   --fmad=false build may not split sums over lanes: 100 cells 0.197 / 0.565 s,
+   even at about 500. */
+#if defined(GC_LU_RECIP) && GC_LU_RECIP
+const int kCoopCells = 24000;
+const bool kCoopAlways = true;      /* without the fused factorisation */
+#else
+const int kCoopCells = 500;
+const bool kCoopAlways = false;
+#endif
+
 struct DevState {
   std::mutex mu;
   bool init = false;
   int sm_count = 0;
-  int mode = RODAS3_PERSISTENT;
+  int mode = kAuto;
   int threads = 128;
   int bps = 0;               /* persistent blocks per SM, 0 = occupancy max */
   int chunk = 0;             /* plain kernels: cells per launch, 0 = env / whole batch */
@@ -88,6 +108,7 @@ int ensure_init(DevState& s, int dev) {
   if (cudaDeviceGetAttribute(&s.sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return -1;
   if (env_is("GCCHEM_B200_MODE", "coop") && rodas3_coop_ok()) s.mode = RODAS3_COOP;
+  else if (env_is("GCCHEM_B200_MODE", "persistent")) s.mode = RODAS3_PERSISTENT;
   else if (env_is("GCCHEM_B200_MODE", "plain_fused")) s.mode = RODAS3_PLAIN_FUSED;
   else if (env_is("GCCHEM_B200_MODE", "plain")) s.mode = RODAS3_PLAIN;
   int t = env_int("GCCHEM_B200_THREADS", 128);
@@ -107,12 +128,19 @@ int ensure_init(DevState& s, int dev) {
   return 0;
 }
 
+/* the kernel that solves nCell cells */
+int auto_mode(const DevState& s, int nCell) {
+  if (s.mode != kAuto) return s.mode;
+  if (!rodas3_coop_ok()) return RODAS3_PERSISTENT;
+  const bool always = kCoopAlways && !rodas3_fused_lu();
+  return always || nCell <= kCoopCells ? RODAS3_COOP : RODAS3_PERSISTENT;
+}
+
 long round_up(long x, long m) { return (x + m - 1) / m * m; }
 
-/* slots the launch of nCell cells uses in `mode` (-1: the device's mode);
-   the cooperative kernel keeps each cell in shared memory and uses none */
-long slots_for(const DevState& s, int nCell, int mode = -1) {
-  if (mode < 0) mode = s.mode;
+/* slots the launch of nCell cells uses in `mode`; the cooperative kernel
+   keeps each cell in shared memory and uses none */
+long slots_for(const DevState& s, int nCell, int mode) {
   if (mode == RODAS3_COOP) return 0;
   const long bytes_per_slot = (long)rodas3_ws_elems() * 8;
   if (mode == RODAS3_PLAIN || mode == RODAS3_PLAIN_FUSED) {
@@ -189,9 +217,7 @@ int launch_on(DevState& s, int nCell, double Tstart, double Tend, double* C,
               int* ISTAT, double* RSTAT, int* IERR, cudaStream_t st,
               int* nfail = nullptr, const double* ATOLr = nullptr,
               const double* RTOLr = nullptr, double* ckpt = nullptr, int ckpt_max = 0) {
-  /* the checkpointing forward of the adjoint runs on the persistent kernel
-     when the cooperative kernel is selected (it stores no checkpoints) */
-  const int mode = (s.mode == RODAS3_COOP && ckpt != nullptr) ? RODAS3_PERSISTENT : s.mode;
+  const int mode = auto_mode(s, nCell);
   const long slots = slots_for(s, nCell, mode);
   if (ensure_ws(s, slots) != 0) return -2;
   Rodas3Launch L;
@@ -209,9 +235,11 @@ int launch_on(DevState& s, int nCell, double Tstart, double Tend, double* C,
   L.ISTAT = ISTAT; L.RSTAT = RSTAT; L.IERR = IERR;
   L.ws = s.ws; L.slots = slots; L.qhead = s.qhead; L.threads = s.threads;
   if (mode == RODAS3_COOP) {
+    /* its two block sizes are 128 and 256 */
+    if (L.threads != 256) L.threads = 128;
     /* resident blocks: SMs x blocks per SM (the occupancy limit, or fewer
        when set_launch asked for fewer) */
-    const int occ = rodas3_coop_blocks_per_sm(s.threads);
+    const int occ = rodas3_coop_blocks_per_sm(L.threads);
     const int bps = (s.bps > 0 && s.bps < occ) ? s.bps : occ;
     if (bps <= 0) return -3;
     return rodas3_coop_launch(&L, s.sm_count * bps, st) == cudaSuccess ? 0 : -3;
@@ -494,7 +522,7 @@ int gcchem_b200_reserve(int nCell) {
   DevState& s = g_dev[d];
   std::lock_guard<std::mutex> lock(s.mu);
   if (ensure_init(s, d) != 0) return -1;
-  return ensure_ws(s, slots_for(s, std::max(nCell, 1)));
+  return ensure_ws(s, slots_for(s, std::max(nCell, 1), auto_mode(s, nCell)));
 }
 
 void gcchem_b200_release(void) {
@@ -546,7 +574,7 @@ long gcchem_b200_workspace_slots(int nCell) {
   DevState& s = g_dev[d];
   std::lock_guard<std::mutex> lock(s.mu);
   if (ensure_init(s, d) != 0) return -1;
-  return slots_for(s, std::max(nCell, 1));
+  return slots_for(s, std::max(nCell, 1), auto_mode(s, nCell));
 }
 
 double gcchem_b200_phase_ms(int phase, long slots, int reps) {

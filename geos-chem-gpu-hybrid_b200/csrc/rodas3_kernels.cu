@@ -774,6 +774,8 @@ static size_t solver_smem(int threads, int sw) {
 
 extern "C" int rodas3_shared_scratch_ok(void) { return SMEM_W_OK ? 1 : 0; }
 
+extern "C" int rodas3_fused_lu(void) { return MECH_FUSED_LU; }
+
 extern "C" int rodas3_max_threads(int sw) {
   if (!sw) return 256;
   const int t = (int)((227 * 1024) / (NVAR * sizeof(double))) / 32 * 32;

@@ -41,6 +41,7 @@ void rodas3_sizes(int* nvar, int* nfix, int* nreact, int* nnz);
 int rodas3_persistent_blocks_per_sm(int threads, int shared_scratch);
 int rodas3_max_threads(int shared_scratch);
 int rodas3_shared_scratch_ok(void);
+int rodas3_fused_lu(void);
 cudaError_t rodas3_launch(const Rodas3Launch* L, cudaStream_t s);
 /* the cooperative kernel (coop.cu): one block of 128 or 256 threads per cell,
    the cell state in shared memory, no workspace */

@@ -108,8 +108,9 @@ void gcchem_b200_sizes(int* nvar, int* nfix, int* nreact, int* nnz);
  * gcchem_b200_set_row_scratch; 0 = default 128);
  * blocks_per_sm: resident blocks the persistent and cooperative grids assume
  * (0 = the occupancy calculator's maximum).  Returns 0, or -1 for invalid
- * values.  With the cooperative kernel selected, the checkpointing forward
- * solve of the adjoint runs on the persistent kernel.  The environment
+ * values.  Until set_launch or the environment names a kernel, every call
+ * takes the cooperative or the persistent one by its number of cells.  The
+ * environment
  * variables GCCHEM_B200_MODE (plain|persistent|plain_fused|coop),
  * GCCHEM_B200_THREADS and GCCHEM_B200_BLOCKS_PER_SM set the defaults. */
 int gcchem_b200_set_launch(int mode, int threads, int blocks_per_sm);
@@ -212,8 +213,8 @@ int gcchem_b200_cost_order(const int* keys, int nCell, int* order, void* stream)
  * comes from its own pool, or a thread that must not call cudaMalloc/cudaFree
  * because they synchronise the whole device.  Same arguments as
  * gcchem_b200_integrate_device, and bit for bit the same per-cell results as
- * its one-thread-per-cell launch (mode 0); the default persistent launch
- * factorises with pivot reciprocals in the FMA build and may differ from it
+ * its one-thread-per-cell launch (mode 0); the default launches
+ * factorise with pivot reciprocals in the FMA build and may differ from it
  * in the last bits.  The solver workspace is a fixed array inside the
  * library's device image, so a call takes at most 256 cells; nCell > 256
  * returns -4 and does nothing.
