@@ -60,35 +60,32 @@
 
 #if MECH_COOP
 
-#if !COOP_SPLIT
-static __constant__ int coop_diag_c[NVAR] = MECH_LU_DIAG_INIT;
-#endif
-
-/* shared-memory layout of one cell (in doubles).  Y0 and Y1 carry the fixed
-   species and the constants of the rate tables behind the NVAR species.
-   The rates A and partials B live in areas that are dead at that time:
-   A of the step's first Fun and B in K1..K3 and S (the stages start later),
-   A of the stages' Fun in S and FCN0 (Fcn0 is read by stages 1 and 2 only;
-   it is formed again at every attempt). */
-#define COOP_MAX2(a, b) ((a) > (b) ? (a) : (b))
-#define COOP_NS COOP_MAX2(COOP_MAX2(NREACT - NVAR, COOP_NBP - 3 * NVAR), 1)
+/* shared memory: the coefficients of the sums, shared by the block's cells,
+   then each cell (in doubles).  V holds the state that Fun and Jac read, with
+   the fixed species and the constants of the rate tables behind it, A the
+   rates, or the Jacobian partials of a part of the columns; X is the vector
+   being formed or solved.  The state and the stage vectors live in registers
+   (thread t of the cell owns species t, t + NT, ..).  G, X, A and RX end in a
+   0 and R in a 1, the operands of missing products. */
 #define SO_G     0
-#define SO_Y0    (SO_G + NNZ)
-#define SO_Y1    (SO_Y0 + COOP_NX)
-#define SO_K     (SO_Y1 + COOP_NX)
-#define SO_S     (SO_K + 3 * NVAR)
-#define SO_FCN0  (SO_S + COOP_NS)
-#define SO_K4    (SO_FCN0 + NVAR)
-#define SO_DFDT  SO_K4              /* read by stages 1 and 2, K4 is written by stage 4 */
-#define SO_R     (SO_K4 + NVAR)
-#define SO_EXTRA (SO_R + NVAR)
-#define SO_END   (SO_EXTRA + COOP_NEXTRA + 1)
-#define COOP_NO  0xFFFFFFFFu
-#define COOP_BARRIER 1
-#define COOP_CHAIN 2
-#define COOP_PW  8                  /* product words of a lane fetched one round ahead */
+#define SO_V     (SO_G + NNZ + 1)
+#define SO_X     (SO_V + COOP_NX)
+#define SO_R     (SO_X + NVAR + 1)
+#define SO_A     (SO_R + NVAR + 1)
+#define SO_RX    (SO_A + NREACT + 1)
+#define SO_RED   (SO_RX + NREACT + COOP_NEXTRA + 1)   /* error sums of up to 8 warps, two ints */
+#define SO_CELL  (SO_RED + 9)
+extern __shared__ __align__(16) unsigned char coop_smem[];
 
-extern __shared__ double sm[];
+/* control bits of the streams (mechanism/coop.py) */
+#define CL_LEAD   1u
+#define CL_FIRST  2u
+#define CL_END    4u
+#define CL_CHAIN  8u
+#define CL_DIAG   16u
+#define CL_SCALED 32u
+#define CL_DIAGS  (1u << 15)       /* factorisation: some lane of the warp has CL_DIAG */
+#define CL_UNIFORM (~(CL_LEAD | CL_DIAG | (7u << 6)))   /* the rest is alike in all lanes */
 
 struct CoopArgs {
   int ncell;
@@ -117,283 +114,310 @@ struct CoopCell {
   CellOpts o;
   CellStat st;
   double T, H;
-  int nsteps, ncons, rej_last, rej_more, newstep, ierr, ysel, attempt;
+  int nsteps, ncons, rej_last, rej_more, newstep, ierr, attempt;
 };
 
-/* ---- rounds --------------------------------------------------------------
-   A program (dest, prod, jvs, lu, fwd, bwd; see mechanism/coop.py) is a list
-   of rounds of at most 256 lanes.  What bounds a round is latency: table
-   words from L2, shared-memory operands, the sum's dependent FMAs, the
-   exchanges and the barrier.  The words of the next round are therefore
-   fetched into registers before the current one runs, and all operands of a
-   lane are loaded before its first FMA. */
-enum { P_DEST, P_PROD, P_JVS, P_LU, P_FWD, P_BWD };
-
-template <int NT>
-struct CoopWords {
-  unsigned int h[256 / NT];
-  unsigned int w[256 / NT][COOP_PW];
+/* ---- warp streams ---------------------------------------------------------
+   What bounds a cell is the instruction stream of its busiest warp: an attempt
+   is ~110 dependent levels of a handful of products per lane, so a level takes
+   as long as one warp needs for its few dozen instructions (6 cycles each: ALU
+   latencies, shared memory, exchanges).  Every warp therefore executes its own
+   list of operations (mechanism/coop.py), whose words hold byte offsets that
+   need no tests, and fetches them COOP_DEPTH operations ahead into registers,
+   across the phases of the attempt (L2 answers after ~320 cycles).  One cell,
+   fullchem, time of an attempt on a B200: rounds of the whole block with words
+   loaded one round ahead 185 us, streams 118 us (256 threads: 107 us).  16,000
+   cells: 0.778 s -> 0.468 s with three cells per block. */
+struct CoopFetch {
+  uint4 q[COOP_DEPTH][2];
 };
 
-template <int NT>
-__device__ __forceinline__ void coop_fetch(CoopWords<NT>& q, int2 r,
-                                           const unsigned int* __restrict__ tab) {
-  const int nl = r.y & 0x3FF, k = (r.y >> 10) & 0x3FF;
-#pragma unroll
-  for (int f = 0; f < 256 / NT; ++f) {
-    const int v = threadIdx.x + f * NT;
-    const bool in = v < nl;
-    q.h[f] = in ? __ldg(tab + r.x + v) : COOP_NO;
-#pragma unroll
-    for (int t = 0; t < COOP_PW; ++t)
-      q.w[f][t] = (in && t < k) ? __ldg(tab + r.x + nl * (1 + t) + v) : COOP_NO;
-  }
+template <bool kShare>
+__device__ __forceinline__ uint4 coop_ld(const uint4* p) {
+  uint4 v;
+  if (kShare)   /* the other cells of the block read the same words soon */
+    asm("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  else
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
-/* KK products of a lane: operands first, then the sum in order.  off: the
-   vector operand's place (V for dest, rates or partials for prod and jvs, the
-   solution for the sweeps); rc: the cell's rate constants */
-template <int PROG, int KK>
-__device__ __forceinline__ double coop_products(double acc, const unsigned int* w, int off,
-                                                const double* __restrict__ rc) {
-  double a[KK], b[KK];
-#pragma unroll
-  for (int t = 0; t < KK; ++t) {
-    const unsigned int x = w[t] == COOP_NO ? 0u : w[t];
-    if (PROG == P_DEST) {
-      const int f0 = x & 0x7FF, f2 = x >> 21;
-      a[t] = f0 < NREACT ? __ldg(rc + f0) : sm[SO_EXTRA + f0 - NREACT];
-      b[t] = sm[off + ((x >> 11) & 0x3FF)];
-      if (f2 != NVAR + NFIX) { a[t] = a[t] * b[t]; b[t] = sm[off + f2]; }
-    } else if (PROG == P_PROD || PROG == P_JVS) {
-      a[t] = __ldg(coop_coef + (x & 0xFFFF));
-      b[t] = sm[off + (x >> 16)];
-    } else {
-      a[t] = sm[SO_G + (x & 0xFFFF)];
-      b[t] = sm[(PROG == P_LU ? SO_G : off) + (x >> 16)];
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < KK; ++t) {
-    if (w[t] != COOP_NO) {
-      if (PROG == P_DEST || PROG == P_PROD || PROG == P_JVS) acc = acc + a[t] * b[t];
-      else acc = acc - a[t] * b[t];
+template <int NT>
+__device__ __forceinline__ int2 coop_segment(int seg) {
+  const int k = seg * (NT / 32) + ((threadIdx.x % NT) >> 5);
+  return NT == 128 ? coop_seg4[k] : coop_seg8[k];
+}
+
+template <int NT>
+__device__ __forceinline__ const uint4* coop_stream(int2 sg) {
+  return reinterpret_cast<const uint4*>(NT == 128 ? coop_words4 : coop_words8) + sg.x +
+         (threadIdx.x & 31);
+}
+
+/* barrier of one cell's threads */
+template <int NT, int NG>
+__device__ __forceinline__ void coop_sync(void) {
+  if (NG == 1) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" :: "r"(1 + (int)threadIdx.x / NT), "n"(NT) : "memory");
+}
+
+/* Shared-memory access by 32-bit address: `cell` is the address of the cell's
+   first array, SO a compile-time place, off a byte offset from a stream. */
+template <int SO>
+__device__ __forceinline__ double coop_get(unsigned int cell, unsigned int off) {
+  double x;
+  asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(x) : "r"(cell + off), "n"(SO * 8));
+  return x;
+}
+template <int SO>
+__device__ __forceinline__ void coop_put(unsigned int cell, unsigned int off, double x) {
+  asm volatile("st.shared.f64 [%0+%1], %2;" :: "r"(cell + off), "n"(SO * 8), "d"(x) : "memory");
+}
+template <int SO>
+__device__ __forceinline__ void coop_put_if(bool p, unsigned int cell, unsigned int off, double x) {
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q st.shared.f64 [%0+%1], %2; }"
+               :: "r"(cell + off), "n"(SO * 8), "d"(x), "r"((unsigned int)p) : "memory");
+}
+
+/* a word that all lanes of the warp hold, as a warp-uniform value: branches on
+   it need no convergence bookkeeping */
+__device__ __forceinline__ unsigned int coop_uniform(unsigned int x) {
+  return __reduce_or_sync(0xFFFFFFFFu, x);
+}
+
+enum { P_RATE, P_DEST, P_PROD, P_JVS, P_LU, P_SWEEP };
+
+/* sum over the lane groups of a warp: the s exchanges that its largest group
+   needs, kept by the lanes whose group is that large (ctl) */
+template <int K>
+__device__ __forceinline__ double coop_exchange(double acc, unsigned int lg) {
+  const double y = __shfl_xor_sync(0xFFFFFFFFu, acc, 1 << K);
+  asm("{ .reg .pred q; setp.gt.u32 q, %1, %2; @q add.f64 %0, %0, %3; }"
+      : "+d"(acc) : "r"(lg), "n"(K), "d"(y));
+  return acc;
+}
+__device__ __forceinline__ double coop_fold(double acc, unsigned int ctl, unsigned int s) {
+  const unsigned int lg = (ctl >> 6) & 7u;
+  if (s > 0) {
+    acc = coop_exchange<0>(acc, lg);
+    if (s > 1) {
+      acc = coop_exchange<1>(acc, lg);
+      if (s > 2) {
+        acc = coop_exchange<2>(acc, lg);
+        if (s > 3) {
+          acc = coop_exchange<3>(acc, lg);
+          if (s > 4) acc = coop_exchange<4>(acc, lg);
+        }
+      }
     }
   }
   return acc;
 }
 
-/* what a program leaves behind: out is the result vector of dest and prod
-   and the place of the solution in the sweeps, v the state of Fun */
-struct CoopOut {
-  int out, v;
-  double ghinv;
-  int* ising;
-};
-
-template <int PROG>
-__device__ __forceinline__ void coop_finish(unsigned int h, double acc, const CoopOut& o) {
-  const int d = h & 0x1FFF;
-  if (PROG == P_DEST) {
-    sm[o.out + d] = acc;
-  } else if (PROG == P_PROD) {
-    sm[o.out + d] = acc - sm[o.out + d] * sm[o.v + d];
-  } else if (PROG == P_JVS) {
-    const int row = (int)((h >> 16) & 0xFFF) - 1;
-    if (row >= 0) {
-      acc = acc + o.ghinv;
-      if (fabs(acc) < DBL_MIN) atomicMin(o.ising, row + 1);
-#if COOP_SPLIT
-      if (h >> 28) sm[SO_R + row] = 1.0 / acc;
-#endif
-    }
-    sm[SO_G + d] = acc;
-  } else if (PROG == P_LU) {
-    const int c = (h >> 16) & 0xFFF;
-#if COOP_SPLIT
-    if (h & (1u << 28)) acc = acc * sm[SO_R + c];
-    if (h & (1u << 29)) sm[SO_R + c] = 1.0 / acc;
-#else
-    if (h & (1u << 28)) acc = acc / sm[SO_G + coop_diag_c[c]];
-#endif
-    sm[SO_G + d] = acc;
-  } else if (PROG == P_FWD) {
-    sm[o.out + d] = acc;
-  } else {
-#if COOP_SPLIT
-    if (!(h >> 28)) acc = acc * sm[SO_R + d];
-#else
-    acc = acc / sm[SO_G + coop_diag_c[d]];
-#endif
-    sm[o.out + d] = acc;
+/* four products ((f0*f1)*f2)*f3 */
+__device__ __forceinline__ void coop_rate_op(unsigned int cell, uint4 a, uint4 b, int j, int step,
+                                             int n) {
+  const unsigned int w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  double f[4][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    f[k][0] = coop_get<SO_RX>(cell, w[2 * k] & 0xFFFFu);
+    f[k][1] = coop_get<SO_V>(cell, w[2 * k] >> 16);
+    f[k][2] = coop_get<SO_V>(cell, w[2 * k + 1] & 0xFFFFu);
+    f[k][3] = coop_get<SO_V>(cell, w[2 * k + 1] >> 16);
   }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    coop_put_if<SO_A>(j + k * step < n, cell, 8 * (j + k * step),
+                      ((f[k][0] * f[k][1]) * f[k][2]) * f[k][3]);
 }
 
-#if COOP_SPLIT
-/* A warp chain: up to 32 rows that depend on one another in turn, one per
-   lane.  The factors are loaded ahead; a step is one exchange and one FMA. */
+/* three products of a destruction sum */
+__device__ __forceinline__ double coop_dest_op(unsigned int cell, double acc, uint4 a, uint4 b) {
+  const unsigned int w[6] = {a.z, a.w, b.x, b.y, b.z, b.w}, u = coop_uniform(a.y & CL_UNIFORM);
+  double f[3], h[3], g[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    f[t] = coop_get<SO_RX>(cell, w[2 * t] & 0xFFFFu);
+    h[t] = coop_get<SO_V>(cell, w[2 * t] >> 16);
+    g[t] = coop_get<SO_V>(cell, w[2 * t + 1]);
+  }
+  if (u & CL_FIRST) acc = 0.0;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) acc = acc + (f[t] * h[t]) * g[t];
+  if (u & CL_END) {
+    acc = coop_fold(acc, a.y, (u >> 9) & 7u);
+    coop_put_if<SO_X>(a.y & CL_LEAD, cell, a.x, acc);
+  }
+  return acc;
+}
+
+/* half of a sum operation: three products, then perhaps the entry's end */
 template <int PROG>
-__device__ __forceinline__ void coop_chain(int m, const unsigned int* __restrict__ tab, int x) {
-  const int lane = threadIdx.x & 31;
-  const int row = (int)__ldg(tab + lane);
-  const unsigned int mask = __ldg(tab + 32 + lane);
-  unsigned int pos[16];
+__device__ __forceinline__ double coop_sum_half(unsigned int cell, unsigned int coef, double acc,
+                                                uint4 q) {
+  const unsigned int w[3] = {q.y, q.z, q.w}, ctl = q.x >> 16, d = q.x & 0xFFFFu;
+  const unsigned int u = coop_uniform(ctl & CL_UNIFORM);
+  double a[3], b[3];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) pos[j] = (2 * j < m) ? __ldg(tab + 64 + 32 * j + lane) : 0u;
-  double acc = (lane < m) ? sm[x + row] : 0.0;
-  const double rr = (PROG == P_BWD && lane < m) ? sm[SO_R + row] : 1.0;
+  for (int t = 0; t < 3; ++t) {
+    a[t] = coop_get<0>(coef, w[t] & 0xFFFFu);
+    b[t] = coop_get<SO_A>(cell, w[t] >> 16);
+  }
+  if (u & CL_FIRST) acc = 0.0;
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    if (16 * c < m) {
-      double l[16];
+  for (int t = 0; t < 3; ++t) acc = acc + a[t] * b[t];
+  if (u & CL_END) {
+    acc = coop_fold(acc, ctl, (u >> 9) & 7u);
+    if (PROG == P_PROD) {
+      const double x = coop_get<SO_X>(cell, d), v = coop_get<SO_V>(cell, d);
+      coop_put_if<SO_X>(ctl & CL_LEAD, cell, d, acc - x * v);
+    } else {
+      coop_put_if<SO_G>(ctl & CL_LEAD, cell, d, acc);
+    }
+  }
+  return acc;
+}
+
+/* level operation of the factorisation (P_LU) or a sweep */
+template <int PROG, int NT, int NG>
+__device__ __forceinline__ double coop_level_op(unsigned int cell, double acc, uint4 qa, uint4 qb) {
+  constexpr int BASE = PROG == P_LU ? SO_G : SO_X;
+  const unsigned int ctl = qa.y, d = qa.x & 0xFFFFu, u = coop_uniform(ctl & CL_UNIFORM);
+  const unsigned int w[6] = {qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#if COOP_SPLIT
+  const double r = coop_get<SO_R>(cell, qa.x >> 16);
+#endif
+  if (u & CL_FIRST) {
+    acc = 0.0;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.shared.f64 %0, [%1+%3]; }"
+                 : "+d"(acc) : "r"(cell + d), "r"(ctl & CL_LEAD), "n"(BASE * 8));
+  }
+#if COOP_SPLIT
+  if (PROG == P_SWEEP && (u & CL_CHAIN)) {
+    /* the warp's lanes own consecutive rows: broadcast, subtract, next */
+    double l[6];
+    const unsigned int j0 = (u >> 15) & 31u, used = (u >> 12) & 7u;
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        l[j] = sm[SO_G + ((pos[8 * c + j / 2] >> (16 * (j & 1))) & 0xFFFF)];
+    for (int t = 0; t < 6; ++t) l[t] = coop_get<SO_G>(cell, w[t]);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (16 * c + j < m) {
-          const double xj = __shfl_sync(0xFFFFFFFFu, PROG == P_BWD ? acc * rr : acc, 16 * c + j);
-          if (mask >> (16 * c + j) & 1u) acc = acc - l[j] * xj;
-        }
+    for (int t = 0; t < 6; ++t) {
+      if (t < used) {
+        const double xj = __shfl_sync(0xFFFFFFFFu, (u & CL_SCALED) ? acc * r : acc, j0 + t);
+        if (w[t] != NNZ * 8) acc = acc - l[t] * xj;
       }
     }
-  }
-  if (lane < m) sm[x + row] = PROG == P_BWD ? acc * rr : acc;
-}
+  } else
 #endif
-
-template <int PROG, int NT>
-__device__ __forceinline__ void coop_rounds(int r0, int r1, const unsigned int* __restrict__ tab,
-                                            int off, const double* __restrict__ rc,
-                                            const CoopOut& o) {
-  CoopWords<NT> nxt;
-  int2 rn = coop_round[r0];
-  coop_fetch<NT>(nxt, rn, tab);
-  for (int r = r0; r < r1; ++r) {
-    const CoopWords<NT> cur = nxt;
-    const int2 rd = rn;
-    if (r + 1 < r1) {
-      rn = coop_round[r + 1];
-      coop_fetch<NT>(nxt, rn, tab);
+  {
+    double a[6], b[6];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      a[t] = coop_get<SO_G>(cell, w[t] & 0xFFFFu);
+      b[t] = coop_get<BASE>(cell, w[t] >> 16);
     }
-    const int nl = rd.y & 0x3FF, k = (rd.y >> 10) & 0x3FF, s = (rd.y >> 20) & 0xF,
-              flags = rd.y >> 24;
-#if COOP_SPLIT
-    if ((PROG == P_FWD || PROG == P_BWD) && (flags & COOP_CHAIN)) {
-      if (threadIdx.x < 32) coop_chain<PROG>(k, tab + rd.x, o.out);
-    } else
-#endif
-    {
+    if (u & (4u << 12)) {                  /* more than three products */
 #pragma unroll
-      for (int f = 0; f < 256 / NT; ++f) {
-        const int v = threadIdx.x + f * NT;
-        if (v < nl) {                       /* whole warps: nl is a multiple of 32 */
-          const unsigned int h = cur.h[f];
-          const int lg = (h >> 13) & 7;
-          const bool lead = h != COOP_NO && (v & ((1 << lg) - 1)) == 0;
-          double acc = 0.0;
-          if (PROG == P_LU && lead) acc = sm[SO_G + (h & 0x1FFF)];
-          if ((PROG == P_FWD || PROG == P_BWD) && lead) acc = sm[o.out + (h & 0x1FFF)];
-          if (k > 4) acc = coop_products<PROG, 8>(acc, cur.w[f], off, rc);
-          else if (k > 2) acc = coop_products<PROG, 4>(acc, cur.w[f], off, rc);
-          else if (k > 0) acc = coop_products<PROG, 2>(acc, cur.w[f], off, rc);
-          for (int t0 = COOP_PW; t0 < k; t0 += 4) {
-            unsigned int w[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-              w[t] = t0 + t < k ? __ldg(tab + rd.x + nl * (1 + t0 + t) + v) : COOP_NO;
-            acc = coop_products<PROG, 4>(acc, w, off, rc);
-          }
-          for (int e = 0; e < s; ++e) {
-            const double y = __shfl_xor_sync(0xFFFFFFFFu, acc, 1 << e);
-            if (e < lg) acc = acc + y;
-          }
-          if (lead) coop_finish<PROG>(h, acc, o);
-        }
+      for (int t = 3; t < 6; ++t) {
+        a[t] = coop_get<SO_G>(cell, w[t] & 0xFFFFu);
+        b[t] = coop_get<BASE>(cell, w[t] >> 16);
       }
+#pragma unroll
+      for (int t = 0; t < 6; ++t) acc = acc - a[t] * b[t];
+    } else {
+#pragma unroll
+      for (int t = 0; t < 3; ++t) acc = acc - a[t] * b[t];
     }
-    if (flags & COOP_BARRIER) __syncthreads();
+  }
+  if (u & CL_END) {
+    acc = coop_fold(acc, ctl, (u >> 9) & 7u);
+#if COOP_SPLIT
+    if (PROG == P_LU) {
+      if (u & CL_DIAGS) {                  /* some lane ends a diagonal */
+        if ((ctl & (CL_LEAD | CL_DIAG)) == (CL_LEAD | CL_DIAG)) coop_put<SO_R>(cell, qa.x >> 16, 1.0 / acc);
+      }
+      if (!(ctl & CL_DIAG)) acc = acc * r;
+    } else {
+      acc = acc * r;
+    }
+#else
+    if ((ctl & (CL_LEAD | CL_SCALED)) == (CL_LEAD | CL_SCALED))
+      acc = acc / coop_get<SO_G>(cell, coop_diag[qa.x >> 19] & ~1);
+#endif
+    coop_put_if<BASE>(ctl & CL_LEAD, cell, d, acc);
+  }
+  if (u >> 20) {
+    for (unsigned int k = u >> 20; k > 0; --k) coop_sync<NT, NG>();
+  }
+  return acc;
+}
+
+/* fetch the first operations of a segment */
+template <int NT, int NG>
+__device__ __forceinline__ void coop_prime(CoopFetch& f, int seg) {
+  const uint4* p = coop_stream<NT>(coop_segment<NT>(seg));
+#pragma unroll
+  for (int d = 0; d < COOP_DEPTH; ++d) {
+    f.q[d][0] = coop_ld<(NG > 1)>(p + d * 64);
+    f.q[d][1] = coop_ld<(NG > 1)>(p + d * 64 + 32);
   }
 }
 
-/* products of four factors (rates A, partials B), one per thread and pass:
-   ((f0*f1)*f2)*f3, absent factors being the constant 1 */
-template <int NT, int N>
-__device__ __forceinline__ void coop_rates(const unsigned short* __restrict__ rec, int v, int out,
-                                           const double* __restrict__ rc) {
-  const ushort4* r4 = reinterpret_cast<const ushort4*>(rec);
-#pragma unroll 4
-  for (int j = threadIdx.x; j < N; j += NT) {
-    const ushort4 f = __ldg(r4 + j);
-    double x = f.x < NREACT ? __ldg(rc + f.x) : sm[SO_EXTRA + f.x - NREACT];
-    x = (x * sm[v + f.y]) * sm[v + f.z];
-    if (f.w != NVAR + NFIX) x = x * sm[v + f.w];
-    sm[out + j] = x;
+/* run a segment; the fetches of its last operations belong to `next`.
+   n: number of products (rates) */
+template <int PROG, int NT, int NG>
+__device__ __forceinline__ void coop_run(unsigned int cell, CoopFetch& f, int seg, int next,
+                                         int n = 0) {
+  const int2 sg = coop_segment<NT>(seg);
+  const uint4* cur = coop_stream<NT>(sg);
+  const uint4* nxt = coop_stream<NT>(coop_segment<NT>(next));
+  const unsigned int coef = (unsigned int)__cvta_generic_to_shared(coop_smem);
+  double acc = 0.0;
+  int j = threadIdx.x % NT;                    /* rates: number of the first product */
+#pragma unroll 1
+  for (int i = COOP_DEPTH; i <= sg.y; i += COOP_DEPTH) {
+    const uint4* p = i < sg.y ? cur + i * 64 : nxt;
+#pragma unroll
+    for (int d = 0; d < COOP_DEPTH; ++d) {
+      const uint4 a = f.q[d][0], b = f.q[d][1];
+      if (PROG == P_RATE) {
+        coop_rate_op(cell, a, b, j, NT, n);
+        j += 4 * NT;
+      } else if (PROG == P_DEST) {
+        acc = coop_dest_op(cell, acc, a, b);
+      } else if (PROG == P_LU || PROG == P_SWEEP) {
+        acc = coop_level_op<PROG, NT, NG>(cell, acc, a, b);
+      } else {
+        acc = coop_sum_half<PROG>(cell, coef, acc, a);
+        acc = coop_sum_half<PROG>(cell, coef, acc, b);
+      }
+      /* into the registers just read: a load into others would be copied at
+         the end of the loop, and the copy would wait for it */
+      f.q[d][0] = coop_ld<(NG > 1)>(p + d * 64);
+      f.q[d][1] = coop_ld<(NG > 1)>(p + d * 64 + 32);
+    }
   }
-}
-
-/* Fun_SPLIT: out = P_VAR - D_VAR*V, rates A at `area`.  The destruction
-   sums need no rates, so they run before the barrier that publishes A. */
-template <int NT>
-__device__ __noinline__ void coop_fun(int v, int out, int area, const double* __restrict__ rc) {
-  CoopOut o;
-  o.out = out; o.v = v; o.ghinv = 0.0; o.ising = nullptr;
-  coop_rates<NT, NREACT>(coop_rate, v, area, rc);
-  coop_rounds<P_DEST, NT>(COOP_R0_DEST, COOP_R1_DEST, coop_w_dest, v, rc, o);
-  __syncthreads();
-  coop_rounds<P_PROD, NT>(COOP_R0_PROD, COOP_R1_PROD, coop_w_prod, area, rc, o);
-}
-
-/* Jac_SP straight into ros_PrepareMatrix's form: G = -JVS, plus ghinv on
-   the diagonal.  KppDecomp's singularity test reads each prepared diagonal
-   before its row is eliminated, so it is taken here: *ising becomes the
-   lowest failing row + 1 (it holds INT_MAX on entry). */
-template <int NT>
-__device__ __forceinline__ void coop_jac_prep(int v, const double* __restrict__ rc, double ghinv,
-                                              int* ising) {
-  CoopOut o;
-  o.out = 0; o.v = v; o.ghinv = ghinv; o.ising = ising;
-  coop_rates<NT, COOP_NBP>(coop_bpart, v, SO_K, rc);
-  __syncthreads();
-  coop_rounds<P_JVS, NT>(COOP_R0_JVS, COOP_R1_JVS, coop_w_jvs, SO_K, rc, o);
-}
-
-/* KppDecomp entry by entry, in levels: G(i,c) - sum L(i,j) U(j,c), times
-   1/U(c,c) (R, FMA build) or over U(c,c) left of the diagonal */
-template <int NT>
-__device__ __forceinline__ void coop_decomp() {
-  CoopOut o;
-  o.out = 0; o.v = 0; o.ghinv = 0.0; o.ising = nullptr;
-  coop_rounds<P_LU, NT>(COOP_R0_LU, COOP_R1_LU, coop_w_lu, SO_G, nullptr, o);
-}
-
-/* KppSolve in place on the vector at x (the caller has synchronised after
-   writing it) */
-template <int NT>
-__device__ __forceinline__ void coop_solve(int x) {
-  CoopOut o;
-  o.out = x; o.v = 0; o.ghinv = 0.0; o.ising = nullptr;
-  coop_rounds<P_FWD, NT>(COOP_R0_FWD, COOP_R1_FWD, coop_w_fwd, x, nullptr, o);
-  coop_rounds<P_BWD, NT>(COOP_R0_BWD, COOP_R1_BWD, coop_w_bwd, x, nullptr, o);
 }
 
 /* load the cell's column and set the integrator state (lane_start of the
    one-thread-per-cell kernels); attempt 1 is the retry: Hstart taken as 0
    and the retry tolerances */
-__device__ __forceinline__ void coop_start(CoopCell& c, const CoopArgs& a, long col,
-                                           int attempt) {
+template <int NT, int NG>
+__device__ __forceinline__ void coop_start(CoopCell& c, const CoopArgs& a, double* sm, double* y,
+                                           long col, int attempt) {
+  const int tid = threadIdx.x % NT;
   c.col = col;
   c.attempt = attempt;
   const double* cc = a.C + col * NSPEC;
   const double* rr = a.RCONST + col * NREACT;
-  for (int i = threadIdx.x; i < COOP_NX; i += blockDim.x) {
-    const double y = i < NSPEC ? cc[i] : coop_ext[i - NSPEC];
-    sm[SO_Y0 + i] = y;
-    if (i >= NVAR) sm[SO_Y1 + i] = y;
-  }
-  for (int i = threadIdx.x; i < COOP_NEXTRA; i += blockDim.x) {
+#pragma unroll
+  for (int m = 0; m < (NVAR + NT - 1) / NT; ++m) y[m] = tid + m * NT < NVAR ? cc[tid + m * NT] : 0.0;
+  for (int i = NVAR + tid; i < COOP_NX; i += NT) sm[SO_V + i] = i < NSPEC ? cc[i] : coop_ext[i - NSPEC];
+  for (int j = tid; j < NREACT; j += NT) sm[SO_RX + j] = rr[j];
+  for (int i = tid; i < COOP_NEXTRA; i += NT) {
     const int j = coop_extra_src[i];
-    sm[SO_EXTRA + i] = j >= 0 ? rr[j] * coop_extra_val[i] : coop_extra_val[i];
+    sm[SO_RX + NREACT + i] = j >= 0 ? rr[j] * coop_extra_val[i] : coop_extra_val[i];
   }
   c.o = decode_options(a.ICNTRL + col * 20, a.RCNTRL + col * 20, a.tstart, a.tend, attempt);
   c.st.nfun = c.st.njac = c.st.nstp = c.st.nacc = 0;
@@ -409,8 +433,7 @@ __device__ __forceinline__ void coop_start(CoopCell& c, const CoopArgs& a, long 
   c.ncons = 0;
   c.rej_last = c.rej_more = 0;
   c.newstep = 1;
-  c.ysel = 0;
-  __syncthreads();
+  coop_sync<NT, NG>();
 }
 
 __device__ __forceinline__ void coop_store_istat(const CoopCell& c, const CoopArgs& a, int add) {
@@ -424,22 +447,25 @@ __device__ __forceinline__ void coop_store_istat(const CoopCell& c, const CoopAr
 /* the end of a solve (lane_end / lane_finish of the other kernels): with the
    retry protocol on, a failed first solve stores its counters and restarts
    from the untouched input column; returns 1 when the cell is finished */
-__device__ __forceinline__ int coop_end(CoopCell& c, const CoopArgs& a) {
+template <int NT, int NG>
+__device__ __forceinline__ int coop_end(CoopCell& c, const CoopArgs& a, double* sm, double* y) {
+  const int tid = threadIdx.x % NT;
   if (a.nfail && c.attempt == 0 && c.ierr < 0) {
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       coop_store_istat(c, a, 0);
       atomicAdd(&a.nfail[0], 1);
     }
-    __syncthreads();
-    coop_start(c, a, c.col, 1);
+    coop_sync<NT, NG>();
+    coop_start<NT, NG>(c, a, sm, y, c.col, 1);
     if (c.ierr == 0) return 0;
   }
   if (c.o.ierr_early == 0) {
-    const double* Y = sm + (c.ysel ? SO_Y1 : SO_Y0);
     double* cc = a.C + c.col * NSPEC;
-    for (int i = threadIdx.x; i < NVAR; i += blockDim.x) cc[i] = Y[i];
+#pragma unroll
+    for (int m = 0; m < (NVAR + NT - 1) / NT; ++m)
+      if (tid + m * NT < NVAR) cc[tid + m * NT] = y[m];
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     coop_store_istat(c, a, c.attempt);
     if (c.attempt && c.ierr < 0) atomicAdd(&a.nfail[1], 1);
     double* rs = a.RSTAT + c.col * 3;
@@ -472,14 +498,15 @@ __device__ __forceinline__ double coop_root(double x) {
    for the block's cell; returns 1 when the cell is finished (c.ierr holds
    IERR).  The statement-level arithmetic is that of step_begin,
    step_prologue, step_factor and step_stages in rodas3_kernels.cu. */
-template <int NT>
-__device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, int* s_ising,
-                                            double* s_err) {
-  const int tid = threadIdx.x;
+template <int NT, int NG>
+__device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, CoopFetch& f,
+                                            unsigned int cell, double* sm, double* y) {
+  const int tid = threadIdx.x % NT;
+  constexpr int NE = (NVAR + NT - 1) / NT;      /* species of a thread */
   const double Tend = a.tend;
   const double dir = (Tend >= a.tstart) ? 1.0 : -1.0;
-  const int y = c.ysel ? SO_Y1 : SO_Y0, ynew = c.ysel ? SO_Y0 : SO_Y1;
-  const double* __restrict__ rc = a.RCONST + c.col * NREACT;
+  double* s_err = sm + SO_RED;
+  int* s_ising = reinterpret_cast<int*>(sm + SO_RED + 8);
 
   if (c.newstep) {
     /* TimeLoop exit tests and the H clamp */
@@ -496,108 +523,162 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, int*
     c.ncons = 0;
   }
 
-  /* Fcn0 [, dFdT] and the Jacobian.  A retried attempt forms them again from
-     the unchanged state (the same values; the counters move once per step):
-     their shared memory holds the stages' rates meanwhile. */
-  coop_fun<NT>(y, SO_FCN0, SO_K, rc);
-  if (!c.o.autonomous) {
-    const double delta = sqrt(ROUNDOFF) * fmaxF(1.0e-6, fabs(c.T));
-    coop_fun<NT>(y, SO_DFDT, SO_K, rc);
-    for (int k = tid; k < NVAR; k += NT)
-      sm[SO_DFDT + k] = (sm[SO_DFDT + k] - sm[SO_FCN0 + k]) / delta;
-  }
-
-  /* ros_PrepareMatrix + KppDecomp */
-  const double ghinv = 1.0 / ((dir * c.H) * 0.5);
-  if (tid == 0) *s_ising = INT_MAX;
-  coop_jac_prep<NT>(y, rc, ghinv, s_ising);
-  const int ising = (*s_ising == INT_MAX) ? 0 : *s_ising;
-  if (ising == 0) coop_decomp<NT>();
-  c.st.ndec += 1;
-  if (ising != 0) {
-    c.st.nsng += 1;
-    c.ncons += 1;
-    __syncthreads();      /* every thread has read *s_ising */
-    if (c.ncons <= 5) { c.H = c.H * 0.5; return 0; }
-    c.ierr = -8;
-    return 1;
-  }
-
-  /* the four stages (per-element operation order of :595-632) */
   const double dH = dir * c.H;
   const double hc1 = 1.0 / dH, hc2 = -1.0 / dH, hc3 = -(8.0 / 3.0) / dH, hc21 = 4.0 / dH;
-  for (int s = 0; s < 4; ++s) {
-    const int x = s < 3 ? SO_K + s * NVAR : SO_K4;
-    if (s >= 2) {
-      /* Ynew = (Y + 2 K1) + 0 K2, then + 1 K3 for stage 4 (Ynew still holds
-         stage 3's value, rounded as the reference's expression rounds it) */
-      for (int k = tid; k < NVAR; k += NT)
-        sm[ynew + k] = s == 2 ? (sm[y + k] + 2.0 * sm[SO_K + k]) + 0.0 * sm[SO_K + NVAR + k]
-                              : sm[ynew + k] + 1.0 * sm[SO_K + 2 * NVAR + k];
-      __syncthreads();
-      coop_fun<NT>(ynew, x, SO_S, rc);
-      c.st.nfun += 1;
-    }
-    for (int k = tid; k < NVAR; k += NT) {
-      double v;
-      if (s == 0) {
-        v = sm[SO_FCN0 + k];
-        if (!c.o.autonomous) v = v + (dH * 0.5) * sm[SO_DFDT + k];
-      } else if (s == 1) {
-        v = sm[SO_FCN0 + k] + hc21 * sm[SO_K + k];
-        if (!c.o.autonomous) v = v + (dH * 1.5) * sm[SO_DFDT + k];
-      } else {
-        v = (sm[x + k] + hc1 * sm[SO_K + k]) + hc2 * sm[SO_K + NVAR + k];
-        if (s == 3) v = v + hc3 * sm[SO_K + 2 * NVAR + k];
+  const double ghinv = 1.0 / (dH * 0.5);
+  if (tid == 0) *s_ising = INT_MAX;
+  double f0[NE], k1[NE], k2[NE], k3[NE], yn[NE];
+
+  /* s = -1: Fcn0, the Jacobian and its factorisation.  A retried attempt
+     forms Fcn0 and the Jacobian again from the unchanged state (the same
+     values; the counters move once per step), so neither is stored.
+     s = 0..3: the stages (per-element operation order of :595-632). */
+#pragma unroll 1
+  for (int s = -1; s < 4; ++s) {
+    if (s == -1 || s >= 2) {
+      /* the state that Fun reads: Y, then Ynew = (Y + 2 K1) + 0 K2, then
+         + 1 K3 (yn still holds stage 3's value, rounded as the reference's
+         expression rounds it) */
+#pragma unroll
+      for (int m = 0; m < NE; ++m) {
+        const int k = tid + m * NT;
+        if (s == -1) yn[m] = y[m];
+        else if (s == 2) yn[m] = (y[m] + 2.0 * k1[m]) + 0.0 * k2[m];
+        else yn[m] = yn[m] + 1.0 * k3[m];
+        if (k < NVAR) sm[SO_V + k] = yn[m];
       }
-      sm[x + k] = v;
+      if (s >= 2) c.st.nfun += 1;
+      coop_sync<NT, NG>();
+      /* Fun_SPLIT: X = P_VAR - D_VAR*V; the destruction sums need no rates,
+         so they run before the barrier that publishes A */
+      coop_run<P_RATE, NT, NG>(cell, f, COOP_SEG_RATE, COOP_SEG_DEST, NREACT);
+      coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_PROD);
+      coop_sync<NT, NG>();
+      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
+      coop_sync<NT, NG>();
     }
-    __syncthreads();
-    coop_solve<NT>(x);
+    if (s == -1) {
+#pragma unroll
+      for (int m = 0; m < NE; ++m) f0[m] = tid + m * NT < NVAR ? sm[SO_X + tid + m * NT] : 0.0;
+      /* Jac_SP straight into ros_PrepareMatrix's form: G = -JVS, a part of
+         the columns at a time, then ghinv on the diagonal.  KppDecomp's
+         singularity test reads each prepared diagonal before its row is
+         eliminated, so it is taken here: *ising becomes the lowest failing
+         row + 1.  Diagonals without updates are final: their reciprocals. */
+#pragma unroll 1
+      for (int q = 0; q < COOP_PARTS; ++q) {
+        const int seg = COOP_SEG_BPART0 + 2 * q;
+        coop_run<P_RATE, NT, NG>(cell, f, seg, seg + 1, COOP_NBP(q));
+        coop_sync<NT, NG>();
+        coop_run<P_JVS, NT, NG>(cell, f, seg + 1, q + 1 < COOP_PARTS ? seg + 2 : COOP_SEG_LU);
+        coop_sync<NT, NG>();
+      }
+#pragma unroll
+      for (int m = 0; m < NE; ++m) {
+        const int k = tid + m * NT;
+        if (k < NVAR) {
+          const int o = __ldg(coop_diag + k);
+          const double g = coop_get<SO_G>(cell, o & ~1) + ghinv;
+          if (fabs(g) < DBL_MIN) atomicMin(s_ising, k + 1);
+          coop_put<SO_G>(cell, o & ~1, g);
+#if COOP_SPLIT
+          if (o & 1) sm[SO_R + k] = 1.0 / g;
+#endif
+        }
+      }
+      coop_sync<NT, NG>();
+      c.st.ndec += 1;
+      if (*s_ising != INT_MAX) {
+        c.st.nsng += 1;
+        c.ncons += 1;
+        coop_prime<NT, NG>(f, COOP_SEG_RATE);
+        coop_sync<NT, NG>();      /* every thread has read *s_ising */
+        if (c.ncons <= 5) { c.H = c.H * 0.5; return 0; }
+        c.ierr = -8;
+        return 1;
+      }
+      /* KppDecomp entry by entry, in levels */
+      coop_run<P_LU, NT, NG>(cell, f, COOP_SEG_LU, COOP_SEG_SWEEP);
+      continue;
+    }
+#pragma unroll
+    for (int m = 0; m < NE; ++m) {
+      const int k = tid + m * NT;
+      if (k < NVAR) {
+        double v;
+        if (s < 2) {
+          v = f0[m];
+          if (s == 1) v = v + hc21 * k1[m];
+          if (!c.o.autonomous) {
+            /* dFdT = (Fun(Y) - Fcn0)/delta: Fun has no explicit time here, so
+               its second evaluation is Fcn0 itself */
+            const double dfdt = (f0[m] - f0[m]) / (sqrt(ROUNDOFF) * fmaxF(1.0e-6, fabs(c.T)));
+            v = v + (s == 0 ? dH * 0.5 : dH * 1.5) * dfdt;
+          }
+        } else {
+          v = (sm[SO_X + k] + hc1 * k1[m]) + hc2 * k2[m];
+          if (s == 3) v = v + hc3 * k3[m];
+        }
+        sm[SO_X + k] = v;
+      }
+    }
+    coop_sync<NT, NG>();
+    coop_run<P_SWEEP, NT, NG>(cell, f, COOP_SEG_SWEEP, s == 0 ? COOP_SEG_SWEEP : COOP_SEG_RATE);
     c.st.nsol += 1;
+    if (s < 3) {
+#pragma unroll
+      for (int m = 0; m < NE; ++m) {
+        const double v = tid + m * NT < NVAR ? sm[SO_X + tid + m * NT] : 0.0;
+        if (s == 0) k1[m] = v;
+        else if (s == 1) k2[m] = v;
+        else k3[m] = v;
+      }
+    }
   }
 
   /* Ynew, Yerr and the scaled error terms in parallel; the WRMS sum over
-     warps, or in species order by thread 0 where the build rounds like the
+     warps, or in species order by one thread where the build rounds like the
      reference */
   const double* atol = c.attempt ? a.ATOLr : a.ATOL;
   const double* rtol = c.attempt ? a.RTOLr : a.RTOL;
   double err = 0.0;
-  for (int i = tid; i < NVAR; i += NT) {
-    const double yi = sm[y + i];
-    const double k1 = sm[SO_K + i], k2 = sm[SO_K + NVAR + i], k3 = sm[SO_K + 2 * NVAR + i],
-                 k4 = sm[SO_K4 + i];
-    const double yn = (((yi + 2.0 * k1) + 0.0 * k2) + 1.0 * k3) + 1.0 * k4;
-    sm[ynew + i] = yn;
-    const double ye = (((0.0 + 0.0 * k1) + 0.0 * k2) + 0.0 * k3) + 1.0 * k4;
-    const double ymax = fmaxF(fabs(yi), fabs(yn));
-    const double scal = c.o.vectortol ? (__ldg(atol + i) + __ldg(rtol + i) * ymax)
-                                      : (__ldg(atol) + __ldg(rtol) * ymax);
-    const double q = ye / scal;
+#pragma unroll
+  for (int m = 0; m < NE; ++m) {
+    const int i = tid + m * NT;
+    if (i < NVAR) {
+      const double yi = y[m];
+      const double k4 = sm[SO_X + i];
+      yn[m] = (((yi + 2.0 * k1[m]) + 0.0 * k2[m]) + 1.0 * k3[m]) + 1.0 * k4;
+      const double ye = (((0.0 + 0.0 * k1[m]) + 0.0 * k2[m]) + 0.0 * k3[m]) + 1.0 * k4;
+      const double ymax = fmaxF(fabs(yi), fabs(yn[m]));
+      const double scal = c.o.vectortol ? (__ldg(atol + i) + __ldg(rtol + i) * ymax)
+                                        : (__ldg(atol) + __ldg(rtol) * ymax);
+      const double q = ye / scal;
 #if COOP_SPLIT
-    err = err + q * q;
+      err = err + q * q;
 #else
-    sm[SO_FCN0 + i] = q;
+      sm[SO_X + i] = q;
 #endif
+    }
   }
 #if COOP_SPLIT
 #pragma unroll
-  for (int e = 16; e > 0; e >>= 1) err = err + __shfl_xor_sync(0xFFFFFFFFu, err, e);
+  for (int k = 16; k > 0; k >>= 1) err = err + __shfl_xor_sync(0xFFFFFFFFu, err, k);
   if ((tid & 31) == 0) s_err[tid >> 5] = err;
-  __syncthreads();
+  coop_sync<NT, NG>();
   err = 0.0;
 #pragma unroll
   for (int w = 0; w < NT / 32; ++w) err = err + s_err[w];
 #else
-  __syncthreads();
+  coop_sync<NT, NG>();
   if (tid == 0) {
     for (int i = 0; i < NVAR; ++i) {
-      const double q = sm[SO_FCN0 + i];
+      const double q = sm[SO_X + i];
       err = err + q * q;
     }
     s_err[0] = err;
   }
-  __syncthreads();
+  coop_sync<NT, NG>();
   err = s_err[0];
 #endif
   err = sqrt(err / (double)NVAR);
@@ -613,13 +694,13 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, int*
     if (a.ckpt && c.st.nacc <= a.ckpt_max) {
       /* checkpoint for the adjoint: the step's starting state and its size */
       double* ck = a.ckpt + (c.col * a.ckpt_max + (c.st.nacc - 1)) * (NVAR + 1);
-      for (int k = tid; k < NVAR; k += NT) ck[k] = sm[y + k];
+#pragma unroll
+      for (int m = 0; m < NE; ++m)
+        if (tid + m * NT < NVAR) ck[tid + m * NT] = y[m];
       if (tid == 0) ck[NVAR] = c.H;
     }
-    if (c.o.clamp) {
-      for (int k = tid; k < NVAR; k += NT) sm[ynew + k] = fmaxF(sm[ynew + k], 0.0);
-    }
-    c.ysel ^= 1;              /* Y = Ynew: the arrays swap roles */
+#pragma unroll
+    for (int m = 0; m < NE; ++m) y[m] = c.o.clamp ? fmaxF(yn[m], 0.0) : yn[m];
     c.T = c.T + dir * c.H;
     hnew = fmaxF(c.o.hmin, fminF(hnew, c.o.hmax));
     if (c.rej_last) hnew = fminF(hnew, c.H);
@@ -638,68 +719,106 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, int*
     if (c.st.nacc >= 1) c.st.nrej += 1;
     c.ncons = 0;
   }
-  __syncthreads();            /* s_err read by all; the clamp is complete */
+  coop_sync<NT, NG>();        /* s_err read by all */
   return 0;
 }
-template <int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) rodas3_coop(CoopArgs a) {
-  __shared__ unsigned int s_pos;
-  __shared__ int s_ising;
-  __shared__ double s_err[NT / 32];
+
+/* NG cells per block, each with NT threads and its own part of the shared
+   memory.  The cells of a block meet at every attempt, so that they read the
+   same stream words at about the same time and share them through L1; in
+   between each synchronises on its own barrier. */
+template <int NT, int NG>
+__global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 256 / NT) rodas3_coop(CoopArgs a) {
+  __shared__ unsigned int s_pos[NG];
+  const int g = NG == 1 ? 0 : threadIdx.x / NT, tid = threadIdx.x % NT;
+  double* sm = reinterpret_cast<double*>(coop_smem) + COOP_NCOEF + g * SO_CELL;
+  const unsigned int cell = (unsigned int)__cvta_generic_to_shared(sm);
+  for (int i = threadIdx.x; i < COOP_NCOEF; i += NT * NG)
+    reinterpret_cast<double*>(coop_smem)[i] = coop_coef[i];
+  if (tid == 0) {
+    sm[SO_G + NNZ] = sm[SO_X + NVAR] = sm[SO_A + NREACT] = sm[SO_RX + NREACT + COOP_NEXTRA] = 0.0;
+    sm[SO_R + NVAR] = 1.0;
+  }
+  __syncthreads();
+  CoopFetch f;
+  coop_prime<NT, NG>(f, COOP_SEG_RATE);
+  CoopCell c;
+  double y[(NVAR + NT - 1) / NT];
+  int have = 0, drained = 0;
   for (;;) {
-    if (threadIdx.x == 0) s_pos = atomicAdd(a.qhead, 1u);
-    __syncthreads();
-    const unsigned int p = s_pos;
-    __syncthreads();          /* s_pos read by all before thread 0 rewrites it */
-    if (p >= (unsigned int)a.ncell) break;
-    CoopCell c;
-    coop_start(c, a, (long)a.order[p], 0);
-    do {
-      if (c.ierr == 0) {
-        while (!coop_attempt<NT>(c, a, &s_ising, s_err)) {}
+    while (!have && !drained) {
+      if (tid == 0) s_pos[g] = atomicAdd(a.qhead, 1u);
+      coop_sync<NT, NG>();
+      const unsigned int p = s_pos[g];
+      coop_sync<NT, NG>();    /* s_pos read by all before it is written again */
+      if (p >= (unsigned int)a.ncell) {
+        drained = 1;
+      } else {
+        coop_start<NT, NG>(c, a, sm, y, (long)a.order[p], 0);
+        have = c.ierr == 0 || !coop_end<NT, NG>(c, a, sm, y);
       }
-    } while (!coop_end(c, a));
-    __syncthreads();          /* the result is stored before the next cell loads */
+    }
+    if (NG > 1) {
+      if (!__syncthreads_or(have)) break;
+    } else if (!have) {
+      break;
+    }
+    if (have && coop_attempt<NT, NG>(c, a, f, cell, sm, y)) {
+      have = !coop_end<NT, NG>(c, a, sm, y);
+      coop_sync<NT, NG>();    /* the result is stored before the next cell loads */
+    }
   }
 }
 
-static size_t coop_smem_bytes(void) { return (size_t)SO_END * sizeof(double); }
+/* cells per block of the shared form */
+#define COOP_NG 3
 
-/* the kernel instance for a block size (128 or 256 threads) */
-static const void* coop_kernel(int threads) {
-  if (threads == 128) return (const void*)rodas3_coop<128, 3>;
-  if (threads == 256) return (const void*)rodas3_coop<256, 2>;
+static size_t coop_smem_bytes(int cells) { return ((size_t)cells * SO_CELL + COOP_NCOEF) * sizeof(double); }
+
+/* the kernel instances: threads per cell (128 or 256), cells per block */
+static const void* coop_kernel(int threads, int cells) {
+  if (threads == 128) return cells == 1 ? (const void*)rodas3_coop<128, 1> : (const void*)rodas3_coop<128, COOP_NG>;
+  if (threads == 256) return (const void*)rodas3_coop<256, 1>;
   return nullptr;
 }
 
-static cudaError_t coop_attr(int threads) {
-  const void* k = coop_kernel(threads);
+static cudaError_t coop_attr(int threads, int cells) {
+  const void* k = coop_kernel(threads, cells);
   if (!k) return cudaErrorInvalidValue;
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)coop_smem_bytes());
+                              (int)coop_smem_bytes(cells));
 }
 
 extern "C" int rodas3_coop_ok(void) {
-  return coop_smem_bytes() <= 227 * 1024 ? 1 : 0;
+  return coop_smem_bytes(1) <= 227 * 1024 ? 1 : 0;
 }
 
-extern "C" size_t rodas3_coop_smem_bytes(void) { return coop_smem_bytes(); }
+extern "C" size_t rodas3_coop_smem_bytes(void) { return coop_smem_bytes(1); }
 
 extern "C" int rodas3_coop_blocks_per_sm(int threads) {
-  if (!rodas3_coop_ok() || coop_attr(threads) != cudaSuccess) return 0;
+  if (!rodas3_coop_ok() || coop_attr(threads, 1) != cudaSuccess) return 0;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, coop_kernel(threads), threads,
-                                                    coop_smem_bytes()) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, coop_kernel(threads, 1), threads,
+                                                    coop_smem_bytes(1)) != cudaSuccess)
     return 0;
   return nb;
 }
 
-/* blocks: resident blocks of the launch (the caller's SM count x blocks per
-   SM, at most one per cell) */
-extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int blocks, cudaStream_t s) {
+/* bps: blocks per SM that the caller allows (0: as many as fit).  Up to two
+   cells per SM run in blocks of their own; larger batches put three in one
+   block, where they share the coefficients and the stream words. */
+extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bps,
+                                          cudaStream_t s) {
   if (!rodas3_coop_ok()) return cudaErrorInvalidValue;
   const int threads = L->threads;
-  const cudaError_t ea = coop_attr(threads);
+  const int occ = rodas3_coop_blocks_per_sm(threads);
+  if (occ <= 0) return cudaErrorInvalidValue;
+  int cells = 1, blocks = sms * (bps > 0 && bps < occ ? bps : occ);
+  if (threads == 128 && bps <= 0 && L->ncell > blocks && coop_smem_bytes(COOP_NG) <= 227 * 1024) {
+    cells = COOP_NG;
+    blocks = sms;
+  }
+  const cudaError_t ea = coop_attr(threads, cells);
   if (ea != cudaSuccess) return ea;
   if (blocks > L->ncell) blocks = L->ncell;
   if (blocks <= 0) return cudaSuccess;
@@ -711,11 +830,13 @@ extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int blocks, cud
   a.qhead = L->qhead; a.nfail = L->nfail; a.ATOLr = L->ATOLr; a.RTOLr = L->RTOLr;
   a.ckpt = L->ckpt; a.ckpt_max = L->ckpt_max;
   cudaMemsetAsync(L->qhead, 0, sizeof(unsigned int), s);
-  const size_t smem = coop_smem_bytes();
-  if (threads == 128)
-    rodas3_coop<128, 3><<<blocks, 128, smem, s>>>(a);
+  const size_t smem = coop_smem_bytes(cells);
+  if (threads == 256)
+    rodas3_coop<256, 1><<<blocks, 256, smem, s>>>(a);
+  else if (cells == 1)
+    rodas3_coop<128, 1><<<blocks, 128, smem, s>>>(a);
   else
-    rodas3_coop<256, 2><<<blocks, 256, smem, s>>>(a);
+    rodas3_coop<128, COOP_NG><<<blocks, 128 * COOP_NG, smem, s>>>(a);
   return cudaGetLastError();
 }
 

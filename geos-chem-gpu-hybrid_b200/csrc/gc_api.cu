@@ -39,20 +39,20 @@ const int kMaxDev = 64;
 /* launch mode until set_launch or GCCHEM_B200_MODE names a kernel: chosen per
    call by the number of cells (auto_mode) */
 const int kAuto = -1;
-/* The cooperative kernel solves a cell in a thirtieth of the time one thread
-   takes, but keeps only a few cells per SM; one thread per cell catches up
-   once the batch fills the GPU.  Full cold steps on a B200, cooperative /
-   persistent: fullchem 1,000 cells 0.069 / 0.549 s, 16,000 cells 0.778 /
-   1.052 s, about even at 24,000.  Without the fused factorisation (synthetic
-   mechanism) the cooperative kernel wins at every size: 1,500 cells 0.050 /
-   0.692 s, 1.01 M / 0.82 M attempts per second at full load.  The
-   --fmad=false build may not split sums over lanes: 100 cells 0.197 / 0.565 s,
-   even at about 500. */
+/* The cooperative kernel solves a cell in a twentieth of the time one thread
+   takes, but keeps only three cells per SM; one thread per cell catches up
+   once the batch fills the GPU several times.  Full cold steps on a B200,
+   cooperative / persistent: fullchem 1,000 cells 0.035 / 0.549 s, 16,000 cells
+   0.468 / 1.052 s, 40,000 cells 1.151 / 1.436 s; at 238,464 cells 2.9 M / 4.6 M
+   attempts per second.  Without the fused factorisation (synthetic mechanism)
+   the cooperative kernel wins at every size: 1,500 cells 0.034 / 0.692 s,
+   1.5 M / 0.8 M attempts per second at full load.  The --fmad=false build may
+   not split sums over lanes: 100 cells 0.108 / 0.553 s, even at about 1,000. */
 #if defined(GC_LU_RECIP) && GC_LU_RECIP
-const int kCoopCells = 24000;
+const int kCoopCells = 64000;
 const bool kCoopAlways = true;      /* without the fused factorisation */
 #else
-const int kCoopCells = 500;
+const int kCoopCells = 1000;
 const bool kCoopAlways = false;
 #endif
 
@@ -237,12 +237,7 @@ int launch_on(DevState& s, int nCell, double Tstart, double Tend, double* C,
   if (mode == RODAS3_COOP) {
     /* its two block sizes are 128 and 256 */
     if (L.threads != 256) L.threads = 128;
-    /* resident blocks: SMs x blocks per SM (the occupancy limit, or fewer
-       when set_launch asked for fewer) */
-    const int occ = rodas3_coop_blocks_per_sm(L.threads);
-    const int bps = (s.bps > 0 && s.bps < occ) ? s.bps : occ;
-    if (bps <= 0) return -3;
-    return rodas3_coop_launch(&L, s.sm_count * bps, st) == cudaSuccess ? 0 : -3;
+    return rodas3_coop_launch(&L, s.sm_count, s.bps, st) == cudaSuccess ? 0 : -3;
   }
   if (rodas3_launch(&L, st) != cudaSuccess) return -3;
   return 0;

@@ -48,7 +48,7 @@ cudaError_t rodas3_launch(const Rodas3Launch* L, cudaStream_t s);
 int rodas3_coop_ok(void);
 size_t rodas3_coop_smem_bytes(void);
 int rodas3_coop_blocks_per_sm(int threads);
-cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int blocks, cudaStream_t s);
+cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bps, cudaStream_t s);
 double rodas3_fp64_peak_tflops(void);
 long rodas3_cost_scratch(int n);
 cudaError_t rodas3_cost_order(const int* keys, int n, int* order,

@@ -210,160 +210,256 @@ def compile_tables(mech: dict):
 
 
 # ---------------------------------------------------------------------------
-# Level programs.
+# Level programs as warp streams.
 #
 # The elimination order of a sparse mechanism is a chain of rows, but its
 # dependencies are shallow: in fullchem (353 species) the forward sweep has 37
 # levels, the backward sweep 33 and the factorisation, taken entry by entry,
-# 62.  Every phase of the solver is therefore stored as a program of rounds.
-# A round is at most LANES_PER_ROUND lanes; a lane belongs to a group of
-# 1, 2, 4 .. 32 consecutive lanes that shares one result, and adds up at most
-# K products of it:
+# 62.  Every phase of the solver is therefore a program of levels; the entries
+# of a level are independent.  An entry is computed by a group of 1, 2, 4 .. 32
+# consecutive lanes that share its products:
 #
 #     acc (lane 0 of the group: the entry's start value) -= A(word.lo)*B(word.hi)
 #
-# after which the group is summed by S butterfly exchanges and lane 0 finishes
-# the entry.  Rounds of one level need no barrier between them.  The build that
-# must round like the reference takes groups of one lane only (each entry's
-# terms stay one left-to-right sum, in the reference's order); the production
-# build splits long sums (up to 327 terms in fullchem).
+# after which the group is summed by butterfly exchanges and lane 0 finishes
+# the entry.  The build that must round like the reference takes groups of one
+# lane (each entry's terms stay one left-to-right sum, in the reference's
+# order); the production build splits long sums (up to 327 terms in fullchem).
+#
+# The generator places the groups on the block's warps and writes one stream
+# per warp: a list of operations of WORDS words per lane, in the order in which
+# the warp executes them.  The addresses of a stream are known in advance, so
+# the kernel fetches operations several ahead of their use.
+#
+# Operands are given as byte offsets in their array (the kernel keeps the cell
+# in shared memory), so that a word needs no arithmetic; a missing operand
+# points at a constant 0 (or 1) behind the array, so that it needs no test.
+#
+#   rate operations   four products (f0 | f1<<16, f2 | f3<<16).  Product k of
+#                     operation i of warp w and lane l is number
+#                     ((i*4 + k)*NW + w)*32 + l.
+#   dest operations   header, control, three products (f0 | f1<<16, f2)
+#   sum operations    two halves of a header and three words (prod, jvs)
+#   level operations  header, control, six words (lu, sweep)
+#
+# Control word, per lane: L_* flags, log2 of the lane's group, exchanges that
+# the warp does (the largest of its groups), products in use, a chain's first
+# step, block barriers after the operation.  A sum's header is its entry's
+# offset | control << 16; a level's is the entry's offset | the offset of its
+# scale in R << 16.
 
-LANES_PER_ROUND = 256
-NO_WORD = 0xFFFFFFFF
-# cost of a round in cycles (round overhead, per product, per exchange): picks
-# how far a level's sums are split
-ROUND_COST, TERM_COST, FOLD_COST = 60, 12, 45
-MAX_TERMS = 16         # most products of one lane where sums are split
+WORDS = 8
+DEPTH = 4              # operations fetched ahead; a segment is a multiple of it
+L_LEAD, L_FIRST, L_END, L_CHAIN, L_DIAG, L_SCALED = 1, 2, 4, 8, 16, 32
+L_DIAGS = 1 << 15      # factorisation: some lane of the warp has L_DIAG
+L_GROUP, L_FOLD, L_USED, L_STEP, L_SYNC = 6, 9, 12, 15, 20
 CHAIN_MAX = 32         # rows of a warp chain (one lane per row)
-BARRIER = 1            # round flag: the block synchronises after the round
-CHAIN = 2              # pseudo round: a warp chain
+# cycles of an operation: fixed part, per product, per exchange, end of an
+# entry (measured latencies on a B200: shared memory 29, FP64 FMA 9, barrier of
+# 128 threads 19; a lone warp issues every ~3 cycles); they only steer how far
+# sums are split
+OP_COST, TERM_COST, FOLD_COST, END_COST = 70, 18, 40, 40
 
 
-def _group(count, k):
-    g = 1
-    while g < 32 and -(-count // g) > k:
-        g *= 2
-    return g
-
-
-def _pack(items, k, split):
-    """Rounds of one level: items [(header, words)] -> [(K, S, lanes)], lanes
-    a list of (header, log2 group, words)."""
+def _lanes(items, k, split):
+    """Warp rounds of one level: [(header, words)] -> lists of at most 32
+    (header, log2 group, words of the lane), groups aligned to their size."""
     sized = []
     for head, words in items:
-        g = _group(len(words), k) if split else 1
+        g = 1
+        while split and g < 32 and -(-len(words) // g) > k:
+            g *= 2
         sized.append((g, -(-len(words) // g), head, words))
-    # aligned groups: wider groups first; alike lanes share a round
     sized.sort(key=lambda x: (-x[0], -x[1]))
-    rounds, lanes, kmax, gmax = [], [], 0, 1
-    for g, per, head, words in sized:
-        if len(lanes) + g > LANES_PER_ROUND:
-            rounds.append((kmax, gmax.bit_length() - 1, lanes))
-            lanes, kmax, gmax = [], 0, 1
-        for q in range(g):
-            lanes.append((head, g.bit_length() - 1, words[q::g]))
-        kmax, gmax = max(kmax, per), max(gmax, g)
+    rounds, lanes = [], []
+    for g, _, head, words in sized:
+        if len(lanes) + g > 32:
+            rounds.append(lanes)
+            lanes = []
+        lanes += [(head, g.bit_length() - 1, words[q::g]) for q in range(g)]
     if lanes:
-        rounds.append((kmax, gmax.bit_length() - 1, lanes))
+        rounds.append(lanes)
     return rounds
 
 
-def _level_rounds(items, split):
+def _cost(lanes, per_op):
+    k = max(len(w) for _, _, w in lanes)
+    s = max(lg for _, lg, _ in lanes)
+    return OP_COST * max(1, -(-k // per_op)) + TERM_COST * k + FOLD_COST * s + END_COST
+
+
+def _place(items, nw, split, per_op):
+    """A level's rounds on nw warps: (warp lists, cost of the longest)."""
     best, cost = None, None
-    for k in (range(1, MAX_TERMS + 1) if split else (1 << 20,)):
-        r = _pack(items, k, split)
-        c = sum(ROUND_COST + TERM_COST * kk + FOLD_COST * ss for kk, ss, _ in r)
-        if cost is None or c < cost:
-            best, cost = r, c
-    return best
+    longest = max([len(w) for _, w in items] + [1])
+    for k in (range(1, min(longest, 40) + 1) if split else (longest,)):
+        warps, load = [[] for _ in range(nw)], [0] * nw
+        for lanes in sorted(_lanes(items, k, split), key=lambda r: -_cost(r, per_op)):
+            w = load.index(min(load))
+            warps[w].append(lanes)
+            load[w] += _cost(lanes, per_op)
+        if cost is None or max(load) < cost:
+            best, cost = warps, max(load)
+    return best, cost
 
 
-class Program:
-    """Rounds and their table words.  A round's words are its headers (one
-    per lane), then K words per lane, lane-contiguous."""
+class Segment:
+    """One phase: per warp a list of operations (32 lanes x WORDS words).
+    `none`: the word of a missing product (for rates and dest two words)."""
 
-    def __init__(self):
-        self.rounds, self.words = [], []
+    def __init__(self, nw, none, head=0):
+        self.nw, self.none, self.head = nw, none, head
+        self.ops = [[] for _ in range(nw)]
+        self.cost = 0
 
-    def level(self, items, split, barrier=True):
-        rs = _level_rounds(items, split)
-        for n, (k, s, lanes) in enumerate(rs):
-            nl = -(-len(lanes) // 32) * 32
-            off = len(self.words)
-            heads = [NO_WORD] * nl
-            cols = [[NO_WORD] * nl for _ in range(k)]
-            for v, (head, lg, words) in enumerate(lanes):
-                heads[v] = head | lg << 13
-                for t, w in enumerate(words):
-                    cols[t][v] = w
-            self.words += heads + [w for c in cols for w in c]
-            self.rounds.append((off, nl, k, s, BARRIER if barrier and n == len(rs) - 1 else 0))
+    def idle(self):
+        if isinstance(self.none, tuple):
+            return list(self.none) * 4 if self.head is None else [self.head, 0] + list(self.none) * 3
+        return [self.head, 0] + [self.none] * 6
+
+    def pad(self, idle=None):
+        for ops in self.ops:
+            while not ops or len(ops) % DEPTH:
+                ops.append([list(idle or self.idle()) for _ in range(32)])
+        return self
+
+    def rates(self, products):
+        for n, words in enumerate(products):
+            v, w = n // 32 % self.nw, n // (32 * self.nw)
+            if w % 4 == 0 and len(self.ops[v]) == w // 4:
+                self.ops[v].append([self.idle() for _ in range(32)])
+            self.ops[v][w // 4][n % 32][w % 4 * 2:w % 4 * 2 + 2] = words
+        return self.pad()
+
+    def _split(self, lanes, per_op):
+        """A warp round as operations: (lane words, header, control) lists."""
+        k = max(len(w) for _, _, w in lanes)
+        s = max(lg for _, lg, _ in lanes)
+        n = max(1, -(-k // per_op))
+        for t in range(n):
+            ctl = (L_FIRST if t == 0 else 0) | (L_END if t == n - 1 else 0) | s << L_FOLD | \
+                min(per_op, k - per_op * t) << L_USED
+            out = []
+            for x in range(32):
+                if x < len(lanes):
+                    (head, flags), lg, words = lanes[x]
+                    w = words[per_op * t:per_op * (t + 1)]
+                    lead = 0 if x % (1 << lg) else L_LEAD
+                    out.append((head, ctl | lead | flags | lg << L_GROUP, w + [self.none] * (per_op - len(w))))
+                else:
+                    out.append((self.head, ctl, [self.none] * per_op))
+            yield out
+
+    def dest(self, items, split):
+        warps, self.cost = _place(items, self.nw, split, 3)
+        for v, rounds in enumerate(warps):
+            for lanes in rounds:
+                for op in self._split(lanes, 3):
+                    self.ops[v].append([[h, c] + [x for w in ws for x in w] for h, c, ws in op])
+        return self.pad()
+
+    def sums(self, items, split):
+        warps, self.cost = _place(items, self.nw, split, 3)
+        idle = [(self.head, 0, [self.none] * 3)] * 32
+        for v, rounds in enumerate(warps):
+            halves = [op for lanes in rounds for op in self._split(lanes, 3)]
+            if len(halves) % 2:
+                halves.append(idle)
+            for a, b in zip(halves[::2], halves[1::2]):
+                self.ops[v].append([[h | (c & 0xFFF) << 16] + w + [g | (d & 0xFFF) << 16] + u
+                                    for (h, c, w), (g, d, u) in zip(a, b)])
+        return self.pad([self.head] + [self.none] * 3 + [self.head] + [self.none] * 3)
+
+    def level(self, items, split):
+        warps, cost = _place(items, self.nw, split, 6)
+        self.cost += cost + 30
+        for v, rounds in enumerate(warps):
+            for lanes in rounds:
+                diags = L_DIAGS if any(flags & L_DIAG for (_, flags), _, _ in lanes) else 0
+                for op in self._split(lanes, 6):
+                    self.ops[v].append([[h, c | diags] + w for h, c, w in op])
+        self._sync()
 
     def chain(self, rows, pos):
-        """A warp chain over `rows`: lane r owns row r; step j broadcasts row
-        j's value and every lane with an entry (r, j) subtracts its term.
-        Words: the rows, the lanes' step masks, then for every two steps the
-        lanes' factor positions (low and high half)."""
+        """A warp chain over `rows` [(header, flags)]: lane r owns row r; step
+        j broadcasts row j's value and every lane with an entry (r, j)
+        subtracts its term."""
         m = len(rows)
-        off = len(self.words)
-        mask = [sum(1 << j for j in range(m) if (r, j) in pos) for r in range(m)]
-        pad = [0] * (32 - m)
-        self.words += list(rows) + pad + mask + pad
-        for j in range(0, m, 2):
-            self.words += [pos.get((r, j), 0) | pos.get((r, j + 1), 0) << 16 for r in range(m)] + pad
-        self.rounds.append((off, 32, m, 0, CHAIN | BARRIER))
+        for j0 in range(0, m, 6):
+            used = min(6, m - j0)
+            ctl = (L_FIRST if j0 == 0 else 0) | (L_END if j0 + used == m else 0) | \
+                used << L_USED | L_CHAIN | j0 << L_STEP
+            op = []
+            for r in range(32):
+                head, flags, lead = rows[r] + (L_LEAD,) if r < m else (self.head, rows[0][1], 0)
+                op.append([head, ctl | lead | flags] +
+                          [pos.get((r, j), self.none & 0xFFFF) if j < m else self.none & 0xFFFF
+                           for j in range(j0, j0 + 6)])
+            self.ops[0].append(op)
+        self.cost += 45 * m + 100
+        self._sync()
+
+    def _sync(self):
+        """A block barrier after everything so far."""
+        for ops in self.ops:
+            if not ops:
+                ops.append([self.idle() for _ in range(32)])
+            for lane in ops[-1]:
+                lane[1] += 1 << L_SYNC
 
 
-def _sweep(n, deps, split, keep_first):
-    """Program of a triangular sweep.  deps[i]: [(column, factor position)] in
-    the reference's order.  Runs of levels with at most two rows become warp
-    chains (at most CHAIN_MAX rows): first one round level subtracts every
-    term whose column lies outside the chain, then one warp walks the chain."""
+def _sweep(seg, n, deps, split, forward):
+    """Levels of a triangular sweep.  deps[i]: [(column, factor position)] in
+    the reference's order.  Runs of levels with very few rows become warp
+    chains (at most CHAIN_MAX rows): first one level subtracts every term whose
+    column lies outside the chain, then one warp walks the chain."""
+    one = 8 * n << 16                    # offset of the constant 1 behind R
+
+    def head(i):
+        return (8 * i | one, 0) if forward else (8 * i | 8 * i << 16, L_SCALED)
+
     lev = [0] * n
-    order = list(range(n)) if keep_first else list(range(n - 1, -1, -1))
+    order = list(range(n)) if forward else list(range(n - 1, -1, -1))
     for i in order:
         lev[i] = max([lev[c] + 1 for c, _ in deps[i]] + [0])
     nlev = max(lev) + 1 if n else 0
-    by = [[i for i in order if lev[i] == l] for l in range(nlev)]
-    prog = Program()
+    by = [[i for i in order if lev[i] == k] for k in range(nlev)]
 
-    def items(rows, skip=()):
-        return [(i, [p | c << 16 for c, p in deps[i] if c not in skip]) for i in rows]
+    def items(rows, skip=(), bulk=False):
+        return [((8 * i | one, 0) if bulk else head(i), [8 * p | 8 * c << 16 for c, p in deps[i] if c not in skip])
+                for i in rows]
 
-    l = 0
-    while l < nlev:
-        e = l
-        if split and (l > 0 or not keep_first):
+    k = 1 if forward else 0              # the forward sweep leaves level 0 as it is
+    while k < nlev:
+        e = k
+        if split:
             rows = 0
             while e < nlev and len(by[e]) <= (4 if e == 0 else 2) and rows + len(by[e]) <= CHAIN_MAX:
                 rows += len(by[e])
                 e += 1
-        if e - l >= 4:
-            rows = [i for k in range(l, e) for i in by[k]]
+        if e - k >= 4:
+            rows = [i for q in range(k, e) for i in by[q]]
             inside = {i: r for r, i in enumerate(rows)}
-            bulk = [it for it in items(rows, inside) if it[1]]
+            bulk = [it for it in items(rows, inside, True) if it[1]]
             if bulk:
-                prog.level([(h | 1 << 28, w) for h, w in bulk], split)
-            prog.chain(rows, {(inside[i], inside[c]): p for i in rows for c, p in deps[i] if c in inside})
-            l = e
-            continue
-        it = items(by[l])
-        if l == 0 and keep_first:
-            it = []                  # the forward sweep leaves level 0 as it is
-        if it:
-            prog.level(it, split)
-        l += 1
-    return prog
+                seg.level(bulk, split)
+            seg.chain([head(i) for i in rows],
+                      {(inside[i], inside[c]): 8 * p for i in rows for c, p in deps[i] if c in inside})
+            k = e
+        else:
+            seg.level(items(by[k]), split)
+            k += 1
 
 
-def level_programs(mech: dict, split: bool):
+def level_programs(mech: dict, split: bool, nw: int):
     """The cooperative kernel's programs, or None for unsupported expression
-    shapes.  split: sums may be divided over lanes (production build)."""
+    shapes.  split: sums may be divided over lanes (production build); nw:
+    warps of the block."""
     if compile_tables(mech) is None:
         return None
     n, nfix, nnz, nreact = mech["nvar"], mech["nfix"], mech["nnz"], mech["nreact"]
     crow, diag, icol, where = mech["lu_crow"], mech["lu_diag"], mech["lu_icol"], mech["lu_where"]
-    if nnz >= 1 << 13 or n >= 1 << 12:
+    if nnz >= (1 << 13) - 1:           # byte offsets of 16 bits
         return None
     extra = {}                 # first factors behind the rate constants: (reaction or
                                # -1, literal), the literal itself or RCT(j)*literal
@@ -374,7 +470,7 @@ def level_programs(mech: dict, split: bool):
         return table.setdefault(value, len(table))
 
     def product(node):
-        """(first, f1, f2, f3): first indexes [RCT | extra], the others
+        """[first, f1, f2, f3]: first indexes [RCT | extra], the others
         [V | FIX | ext]; missing factors are the constant 1, whose product
         is exact.  A leading RCT(j)*literal is formed once per cell."""
         fs = []
@@ -437,8 +533,26 @@ def level_programs(mech: dict, split: bool):
 
     try:
         rate = [product(e) for e in mech["rates"]]
-        bmap = {m: k for k, (m, _) in enumerate(mech["jac_b"])}
-        bpart = [product(e) for _, e in mech["jac_b"]]
+        # partials B: each feeds one column of the Jacobian only, so they are
+        # formed for a part of the columns at a time, as many as the rates'
+        # scratch array holds
+        col_of = {}
+        for p, e in enumerate(mech["jvs"]):
+            for b in codegen._refs(e, "b"):
+                if col_of.setdefault(b, icol[p]) != icol[p]:
+                    raise Unsupported("partial of two columns")
+        bexpr = dict(mech["jac_b"])
+        parts, part_of = [[]], {}
+        for c in range(n):
+            mine = sorted(b for b, k in col_of.items() if k == c)
+            if len(parts[-1]) + len(mine) > nreact:
+                parts.append([])
+            part_of[c] = len(parts) - 1
+            parts[-1] += mine
+        bmap = {b: k for part in parts for k, b in enumerate(part)}
+        if max(len(part) for part in parts) > nreact:
+            raise Unsupported("column with too many partials")
+        bpart = [[product(bexpr[b]) for b in part] for part in parts]
         dest = []
         for i, e in enumerate(mech["dest"]):
             words = []
@@ -455,33 +569,41 @@ def level_programs(mech: dict, split: bool):
     except (Unsupported, KeyError):
         return None
     nx = n + nfix + len(ext)
-    nrx = nreact + len(extra)
-    if nx >= 1 << 10 or nrx >= 1 << 11 or len(bpart) >= 1 << 16:
+    zero = 8 * (nreact + len(extra))     # the constant 0 behind [RCT | extra]
+    one = 8 * (n + nfix)
+    if max(8 * nx, zero, 8 * len(coef)) >= 1 << 16:
         return None
-    pd = Program()
-    pd.level([(i, [f[0] | f[1] << 11 | f[2] << 21 for f in w]) for i, w in dest], split, False)
-    pp = Program()
-    pp.level(prod, split)
-    # -Jac0 (the coefficients carry the sign), ghinv on the diagonal; bit 28:
-    # a diagonal without updates, whose reciprocal is formed here
+
+    def words4(f):
+        return [8 * f[0] | 8 * f[1] << 16, 8 * f[2] | 8 * f[3] << 16]
+
+    def dword(f):          # (f0*f1)*f2, with the constant 1 in the middle of k*v
+        p, q = (f[2], f[1]) if f[2] == n + nfix else (f[1], f[2])
+        return (8 * f[0] | 8 * p << 16, 8 * q)
+
+    def scaled_words(words):
+        return [8 * (w & 0xFFFF) | 8 * (w >> 16) << 16 for w in words]
+
+    no_rate, no_dest, no_sum = (zero | one << 16, one | one << 16), (zero | one << 16, one), 8 * nreact << 16
+    segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
+            "dest": Segment(nw, no_dest).dest([((8 * i, 0), [dword(f) for f in w]) for i, w in dest], split),
+            "prod": Segment(nw, no_sum).sums([((8 * i, 0), scaled_words(w)) for i, w in prod], split)}
+    # KppDecomp entry by entry: G(i,c) = G(i,c) - sum L(i,j) U(j,c), and for
+    # c < i the product with 1/U(c,c); an entry's level is one above those of
+    # the factors (and of the pivot) that it reads
+    row_of = mech["lu_irow"]
     upd = [[] for _ in range(nnz)]
     for i in range(n):
         for kk in range(crow[i], diag[i]):
             j = icol[kk]
             for jj in range(diag[j] + 1, crow[j + 1]):
                 upd[where[(i, icol[jj])]].append((kk, jj))
-    row_of = mech["lu_irow"]
-    pj = Program()
-    items = []
-    for p in range(nnz):
-        h = p
-        if p == diag[row_of[p]]:
-            h |= (row_of[p] + 1) << 16 | (0 if upd[p] else 1 << 28)
-        items.append((h, jvs[p]))
-    pj.level(items, split)
-    # KppDecomp entry by entry: G(i,c) = G(i,c) - sum L(i,j) U(j,c), and for
-    # c < i the product with 1/U(c,c); an entry's level is one above those of
-    # the factors (and of the pivot) that it reads
+    # -Jac0 (the coefficients carry the sign); the kernel adds ghinv to the
+    # diagonal and forms the reciprocals of the diagonals without updates
+    for q, part in enumerate(bpart):
+        segs[f"bpart{q}"] = Segment(nw, no_rate, None).rates([words4(f) for f in part])
+        segs[f"jvs{q}"] = Segment(nw, no_sum).sums(
+            [((8 * p, 0), scaled_words(jvs[p])) for p in range(nnz) if part_of[icol[p]] == q], split)
     elev = [0] * nnz
     for i in range(n):
         for p in range(crow[i], crow[i + 1]):
@@ -490,63 +612,67 @@ def level_programs(mech: dict, split: bool):
             if c < i:
                 lv = max(lv, elev[diag[c]] + 1)
             elev[p] = lv
-    pl = Program()
-    for l in range(1, max(elev) + 1):
+    none = 8 * nnz | 8 * nnz << 16       # the constant 0 behind G, times itself
+    lu = segs["lu"] = Segment(nw, none, 8 * nnz | 8 * n << 16)
+    for k in range(1, max(elev) + 1):
         items = []
         for p in range(nnz):
-            if elev[p] == l:
+            if elev[p] == k:
                 i, c = row_of[p], icol[p]
-                h = p | c << 16 | (1 << 28 if c < i else (1 << 29 if c == i else 0))
-                items.append((h, [a | b << 16 for a, b in upd[p]]))
-        pl.level(items, split)
-    lower = [[(icol[p], p) for p in range(crow[i], diag[i])] for i in range(n)]
-    upper = [[(icol[p], p) for p in range(diag[i] + 1, crow[i + 1])] for i in range(n)]
-    return {"rate": rate, "bpart": bpart, "extra": extra, "ext": ext, "coef": coef, "nx": nx,
-            "dest": pd, "prod": pp, "jvs": pj, "lu": pl,
-            "fwd": _sweep(n, lower, split, True), "bwd": _sweep(n, upper, split, False)}
-
-
-PROGRAMS = ("dest", "prod", "jvs", "lu", "fwd", "bwd")
+                head = (8 * p | 8 * (c if c <= i else n) << 16, L_SCALED if c < i else L_DIAG if c == i else 0)
+                items.append((head, [8 * a | 8 * b << 16 for a, b in upd[p]]))
+        lu.level(items, split)
+    sweep = segs["sweep"] = Segment(nw, 8 * nnz | 8 * n << 16, 8 * n | 8 * n << 16)
+    _sweep(sweep, n, [[(icol[p], p) for p in range(crow[i], diag[i])] for i in range(n)], split, True)
+    _sweep(sweep, n, [[(icol[p], p) for p in range(diag[i] + 1, crow[i + 1])] for i in range(n)], split, False)
+    lu.pad(), sweep.pad()
+    return {"segs": segs, "parts": len(parts), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
+            "nbp": [len(part) for part in parts],
+            "diag": [(8 * diag[i], not upd[diag[i]]) for i in range(n)]}
 
 
 def coop_inc(mech: dict) -> str:
     """coop.inc: MECH_COOP and, when the programs exist, their C arrays for
-    both builds (COOP_SPLIT), included by one translation unit."""
+    both builds (COOP_SPLIT) and both block sizes, included by one translation
+    unit."""
     t = compile_tables(mech)
-    progs = None if t is None else {sp: level_programs(mech, sp) for sp in (False, True)}
-    if t is None or progs[True] is None:
+    if t is None or level_programs(mech, True, 4) is None:
         return "/* no cooperative-kernel tables: unsupported expression shape */\n" \
                "#define MECH_COOP 0\n"
 
-    def arr(ctype, name, vals, align="", space="__device__ const"):
+    def arr(ctype, name, vals, space="__device__ const"):
         body = ",".join(str(v) for v in vals) if vals else "0"
-        return f"static {space} {align}{ctype} {name}[{max(len(vals), 1)}] = {{{body}}};"
+        return f"static {space} {ctype} {name}[{max(len(vals), 1)}] = {{{body}}};"
 
-    def doubles(name, table):
-        return arr("double", name, [repr(float(v)) for v in table])
+    def doubles(name, vals):
+        return arr("double", name, [repr(float(v)) for v in vals] or [0.0])
 
     lines = ["/* generated cooperative-kernel tables; do not edit */", "#pragma once",
-             "#define MECH_COOP 1", f"#define COOP_NUPD {len(t['upd'])}"]
-    for sp in (False, True):
-        p = progs[sp]
-        lines.append("#if COOP_SPLIT" if sp else "#if !COOP_SPLIT")
-        lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
-                  f"#define COOP_NEXTRA {len(p['extra'])}", f"#define COOP_NCOEF {len(p['coef'])}",
-                  f"#define COOP_NBP {len(p['bpart'])}",
-                  doubles("coop_ext", p["ext"]),
-                  arr("int", "coop_extra_src", [j for j, _ in p["extra"]]),
-                  doubles("coop_extra_val", [v for _, v in p["extra"]] or [0.0]),
-                  doubles("coop_coef", p["coef"]),
-                  arr("unsigned short", "coop_rate", [x for f in p["rate"] for x in f], "__align__(8) "),
-                  arr("unsigned short", "coop_bpart", [x for f in p["bpart"] for x in f], "__align__(8) ")]
-        rounds = []
-        for name in PROGRAMS:
-            pr = p[name]
-            lines.append(f"#define COOP_R0_{name.upper()} {len(rounds)}")
-            rounds += pr.rounds
-            lines.append(f"#define COOP_R1_{name.upper()} {len(rounds)}")
-            lines.append(arr("unsigned int", f"coop_w_{name}", [f"{w}u" for w in pr.words]))
-        body = ",".join("{%d,%d}" % (off, nl | k << 10 | s << 20 | f << 24) for off, nl, k, s, f in rounds)
-        lines.append(f"static __constant__ int2 coop_round[{len(rounds)}] = {{{body}}};")
+             "#define MECH_COOP 1", f"#define COOP_NUPD {len(t['upd'])}", f"#define COOP_DEPTH {DEPTH}"]
+    for split in (False, True):
+        lines.append("#if COOP_SPLIT" if split else "#if !COOP_SPLIT")
+        for nw in (4, 8):
+            p = level_programs(mech, split, nw)
+            if nw == 4:
+                lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
+                          f"#define COOP_NEXTRA {len(p['extra'])}", f"#define COOP_PARTS {p['parts']}",
+                          "#define COOP_NSEG %d" % len(p["segs"]),
+                          doubles("coop_ext", p["ext"]),
+                          arr("int", "coop_extra_src", [j for j, _ in p["extra"]]),
+                          doubles("coop_extra_val", [v for _, v in p["extra"]]),
+                          f"#define COOP_NCOEF {len(p['coef'])}", doubles("coop_coef", p["coef"]),
+                          "#define COOP_NBP(q) (%s)" % " : ".join(
+                              [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),
+                          arr("int", "coop_diag", [o | (e and 1) for o, e in p["diag"]])]
+                lines += [f"#define COOP_SEG_{name.upper()} {k}" for k, name in enumerate(p["segs"])]
+            words, where = [], []
+            for seg in p["segs"].values():
+                for ops in seg.ops:
+                    where.append("{%d,%d}" % (len(words) // 4, len(ops)))
+                    for op in ops:                   # first four words of the lanes, then the others
+                        words += [x for lane in op for x in lane[:4]] + [x for lane in op for x in lane[4:]]
+            lines.append(f"static __constant__ int2 coop_seg{nw}[{len(where)}] = {{{','.join(where)}}};")
+            lines.append(arr("unsigned int", f"coop_words{nw}", [f"{w}u" for w in words],
+                             "__device__ const __align__(16)"))
         lines.append("#endif")
     return "\n".join(lines) + "\n"
