@@ -61,31 +61,38 @@
 #if MECH_COOP
 
 /* shared memory: the coefficients of the sums, shared by the block's cells,
-   then each cell (in doubles).  V holds the state that Fun and Jac read, with
-   the fixed species and the constants of the rate tables behind it, A the
-   rates, or the Jacobian partials of a part of the columns; X is the vector
-   being formed or solved.  The state and the stage vectors live in registers
-   (thread t of the cell owns species t, t + NT, ..).  G, X, A and RX end in a
-   0 and R in a 1, the operands of missing products. */
-#define SO_G     0
-#define SO_V     (SO_G + NNZ + 1)
-#define SO_X     (SO_V + COOP_NX)
-#define SO_R     (SO_X + NVAR + 1)
-#define SO_A     (SO_R + NVAR + 1)
-#define SO_RX    (SO_A + NREACT + 1)
-#define SO_RED   (SO_RX + NREACT + COOP_NEXTRA + 1)   /* error sums of up to 8 warps, two ints */
-#define SO_CELL  (SO_RED + 9)
+   then each cell (in doubles).  G holds the factors, the tail block, the
+   inverses of the sweeps' parts, -1/U(i,i), -1 and 0 (see mechanism/coop.py); V the state that
+   Fun and Jac read, with the fixed species and the constants of the rate
+   tables behind it; A the rates, or the Jacobian partials of a part of the
+   columns; X [vector | 0 | second place].  The state and the stage vectors
+   live in registers (thread t of the cell owns species t, t + NT, ..).  A and
+   RX end in a 0, the operand of missing products.  B is 16-byte aligned (as the
+   cells and COOP_NCOEF are even), for loads of two products. */
+template <int NT>
+struct CoopAt {
+  static constexpr int ZERO = NT == 128 ? COOP_NG4 : COOP_NG8;   /* index of 0 in G */
+  static constexpr int RECIP = ZERO - 1 - NVAR;                  /* of -1/U(0,0) */
+  static constexpr int G = 0;
+  static constexpr int V = G + ZERO + 1;
+  static constexpr int X = V + COOP_NX;
+  static constexpr int A = X + 2 * NVAR + 2;
+  static constexpr int RX = A + NREACT + 1;
+  static constexpr int B = (RX + NREACT + COOP_NEXTRA + 2) / 2 * 2;   /* products of the long sums */
+  static constexpr int RED = B + COOP_BUFFER;   /* error sums of up to 8 warps, two ints */
+  static constexpr int CELL = (RED + 10) / 2 * 2;
+};
 extern __shared__ __align__(16) unsigned char coop_smem[];
 
 /* control bits of the streams (mechanism/coop.py) */
 #define CL_LEAD   1u
 #define CL_FIRST  2u
 #define CL_END    4u
-#define CL_CHAIN  8u
+#define CL_START  8u
 #define CL_DIAG   16u
 #define CL_SCALED 32u
-#define CL_DIAGS  (1u << 15)       /* factorisation: some lane of the warp has CL_DIAG */
-#define CL_UNIFORM (~(CL_LEAD | CL_DIAG | (7u << 6)))   /* the rest is alike in all lanes */
+#define CL_DIAGS  (1u << 15)       /* some lane of the warp has CL_DIAG */
+#define CL_UNIFORM (CL_FIRST | CL_END | ~0u << 9)   /* alike in all lanes */
 
 struct CoopArgs {
   int ncell;
@@ -118,16 +125,16 @@ struct CoopCell {
 };
 
 /* ---- warp streams ---------------------------------------------------------
-   What bounds a cell is the instruction stream of its busiest warp: an attempt
-   is ~110 dependent levels of a handful of products per lane, so a level takes
-   as long as one warp needs for its few dozen instructions (6 cycles each: ALU
-   latencies, shared memory, exchanges).  Every warp therefore executes its own
-   list of operations (mechanism/coop.py), whose words hold byte offsets that
-   need no tests, and fetches them COOP_DEPTH operations ahead into registers,
-   across the phases of the attempt (L2 answers after ~320 cycles).  One cell,
-   fullchem, time of an attempt on a B200: rounds of the whole block with words
-   loaded one round ahead 185 us, streams 118 us (256 threads: 107 us).  16,000
-   cells: 0.778 s -> 0.468 s with three cells per block. */
+   What bounds a cell is the instruction stream of its busiest warp: a level
+   takes as long as one warp needs for its operations (~100 instructions of ~6
+   cycles each: ALU latencies, shared memory, exchanges).  Every warp therefore
+   executes its own list of operations (mechanism/coop.py), whose words hold
+   offsets that need no tests, and fetches them COOP_DEPTH operations ahead into
+   registers, across the phases of the attempt (L2 answers after ~320 cycles);
+   and the programs have few levels.  One cell, fullchem, time of an attempt on
+   a B200: rounds of the whole block with words loaded one round ahead 185 us;
+   streams 118 us; with inverses of the sweeps' parts and of the tail block
+   (13 + 9 levels instead of 61 + 69) 86 us. */
 struct CoopFetch {
   uint4 q[COOP_DEPTH][2];
 };
@@ -186,7 +193,7 @@ __device__ __forceinline__ unsigned int coop_uniform(unsigned int x) {
   return __reduce_or_sync(0xFFFFFFFFu, x);
 }
 
-enum { P_RATE, P_DEST, P_PROD, P_JVS, P_LU, P_SWEEP };
+enum { P_RATE, P_BUFD, P_DEST, P_PROD, P_BUFP, P_JVS, P_ONE, P_LU, P_SWEEP };
 
 /* sum over the lane groups of a warp: the s exchanges that its largest group
    needs, kept by the lanes whose group is that large (ctl) */
@@ -216,45 +223,46 @@ __device__ __forceinline__ double coop_fold(double acc, unsigned int ctl, unsign
 }
 
 /* four products ((f0*f1)*f2)*f3 */
+template <int NT, int OUT>
 __device__ __forceinline__ void coop_rate_op(unsigned int cell, uint4 a, uint4 b, int j, int step,
                                              int n) {
   const unsigned int w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   double f[4][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    f[k][0] = coop_get<SO_RX>(cell, w[2 * k] & 0xFFFFu);
-    f[k][1] = coop_get<SO_V>(cell, w[2 * k] >> 16);
-    f[k][2] = coop_get<SO_V>(cell, w[2 * k + 1] & 0xFFFFu);
-    f[k][3] = coop_get<SO_V>(cell, w[2 * k + 1] >> 16);
+    f[k][0] = coop_get<CoopAt<NT>::RX>(cell, w[2 * k] & 0xFFFFu);
+    f[k][1] = coop_get<CoopAt<NT>::V>(cell, w[2 * k] >> 16);
+    f[k][2] = coop_get<CoopAt<NT>::V>(cell, w[2 * k + 1] & 0xFFFFu);
+    f[k][3] = coop_get<CoopAt<NT>::V>(cell, w[2 * k + 1] >> 16);
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    coop_put_if<SO_A>(j + k * step < n, cell, 8 * (j + k * step),
+    coop_put_if<OUT>(j + k * step < n, cell, 8 * (j + k * step),
                       ((f[k][0] * f[k][1]) * f[k][2]) * f[k][3]);
 }
 
 /* three products of a destruction sum */
+template <int NT>
 __device__ __forceinline__ double coop_dest_op(unsigned int cell, double acc, uint4 a, uint4 b) {
   const unsigned int w[6] = {a.z, a.w, b.x, b.y, b.z, b.w}, u = coop_uniform(a.y & CL_UNIFORM);
   double f[3], h[3], g[3];
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
-    f[t] = coop_get<SO_RX>(cell, w[2 * t] & 0xFFFFu);
-    h[t] = coop_get<SO_V>(cell, w[2 * t] >> 16);
-    g[t] = coop_get<SO_V>(cell, w[2 * t + 1]);
+    f[t] = coop_get<CoopAt<NT>::RX>(cell, w[2 * t] & 0xFFFFu);
+    h[t] = coop_get<CoopAt<NT>::V>(cell, w[2 * t] >> 16);
+    g[t] = coop_get<CoopAt<NT>::V>(cell, w[2 * t + 1]);
   }
   if (u & CL_FIRST) acc = 0.0;
 #pragma unroll
   for (int t = 0; t < 3; ++t) acc = acc + (f[t] * h[t]) * g[t];
   if (u & CL_END) {
-    acc = coop_fold(acc, a.y, (u >> 9) & 7u);
-    coop_put_if<SO_X>(a.y & CL_LEAD, cell, a.x, acc);
+    coop_put_if<CoopAt<NT>::X>(a.y & CL_LEAD, cell, a.x, acc);
   }
   return acc;
 }
 
 /* half of a sum operation: three products, then perhaps the entry's end */
-template <int PROG>
+template <int PROG, int NT>
 __device__ __forceinline__ double coop_sum_half(unsigned int cell, unsigned int coef, double acc,
                                                 uint4 q) {
   const unsigned int w[3] = {q.y, q.z, q.w}, ctl = q.x >> 16, d = q.x & 0xFFFFu;
@@ -263,87 +271,83 @@ __device__ __forceinline__ double coop_sum_half(unsigned int cell, unsigned int 
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
     a[t] = coop_get<0>(coef, w[t] & 0xFFFFu);
-    b[t] = coop_get<SO_A>(cell, w[t] >> 16);
+    b[t] = coop_get<CoopAt<NT>::A>(cell, w[t] >> 16);
   }
   if (u & CL_FIRST) acc = 0.0;
 #pragma unroll
   for (int t = 0; t < 3; ++t) acc = acc + a[t] * b[t];
   if (u & CL_END) {
-    acc = coop_fold(acc, ctl, (u >> 9) & 7u);
+    if (PROG == P_JVS) acc = coop_fold(acc, ctl, (u >> 9) & 7u);
     if (PROG == P_PROD) {
-      const double x = coop_get<SO_X>(cell, d), v = coop_get<SO_V>(cell, d);
-      coop_put_if<SO_X>(ctl & CL_LEAD, cell, d, acc - x * v);
+      const double x = coop_get<CoopAt<NT>::X>(cell, d), v = coop_get<CoopAt<NT>::V>(cell, d);
+      coop_put_if<CoopAt<NT>::X>(ctl & CL_LEAD, cell, d, acc - x * v);
     } else {
-      coop_put_if<SO_G>(ctl & CL_LEAD, cell, d, acc);
+      coop_put_if<CoopAt<NT>::G>(ctl & CL_LEAD, cell, d, acc);
     }
   }
   return acc;
 }
 
-/* level operation of the factorisation (P_LU) or a sweep */
+/* four entries of one product */
+template <int NT, int OUT>
+__device__ __forceinline__ void coop_one_op(unsigned int cell, unsigned int coef, uint4 a, uint4 b) {
+  const unsigned int w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  double f[4], g[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    f[k] = coop_get<0>(coef, w[2 * k] >> 16);
+    g[k] = coop_get<CoopAt<NT>::A>(cell, w[2 * k + 1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned int d = w[2 * k] & 0xFFFFu;
+    coop_put_if<OUT>(d != 0xFFFFu, cell, d, f[k] * g[k]);
+  }
+}
+
+/* level operation of the factorisation (P_LU) or a sweep; operands are element
+   indices */
 template <int PROG, int NT, int NG>
 __device__ __forceinline__ double coop_level_op(unsigned int cell, double acc, uint4 qa, uint4 qb) {
-  constexpr int BASE = PROG == P_LU ? SO_G : SO_X;
-  const unsigned int ctl = qa.y, d = qa.x & 0xFFFFu, u = coop_uniform(ctl & CL_UNIFORM);
+  using L = CoopAt<NT>;
+  constexpr int BASE = PROG == P_LU ? L::G : L::X;
+  const unsigned int ctl = qa.y, d = 8u * (qa.x & 0xFFFFu), e = 8u * (qa.x >> 16);
+  const unsigned int u = coop_uniform(ctl & CL_UNIFORM);
   const unsigned int w[6] = {qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#if COOP_SPLIT
-  const double r = coop_get<SO_R>(cell, qa.x >> 16);
-#endif
+  double a[6], b[6];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    a[t] = coop_get<L::G>(cell, 8u * (w[t] & 0xFFFFu));
+    b[t] = coop_get<BASE>(cell, 8u * (w[t] >> 16));
+  }
   if (u & CL_FIRST) {
     acc = 0.0;
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.shared.f64 %0, [%1+%3]; }"
-                 : "+d"(acc) : "r"(cell + d), "r"(ctl & CL_LEAD), "n"(BASE * 8));
+                 : "+d"(acc) : "r"(cell + d), "r"(ctl & CL_START), "n"(BASE * 8));
   }
-#if COOP_SPLIT
-  if (PROG == P_SWEEP && (u & CL_CHAIN)) {
-    /* the warp's lanes own consecutive rows: broadcast, subtract, next */
-    double l[6];
-    const unsigned int j0 = (u >> 15) & 31u, used = (u >> 12) & 7u;
+  if (u & (4u << 12)) {                    /* more than three products */
 #pragma unroll
-    for (int t = 0; t < 6; ++t) l[t] = coop_get<SO_G>(cell, w[t]);
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      if (t < used) {
-        const double xj = __shfl_sync(0xFFFFFFFFu, (u & CL_SCALED) ? acc * r : acc, j0 + t);
-        if (w[t] != NNZ * 8) acc = acc - l[t] * xj;
-      }
+    for (int t = 3; t < 6; ++t) {
+      a[t] = coop_get<L::G>(cell, 8u * (w[t] & 0xFFFFu));
+      b[t] = coop_get<BASE>(cell, 8u * (w[t] >> 16));
     }
-  } else
-#endif
-  {
-    double a[6], b[6];
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      a[t] = coop_get<SO_G>(cell, w[t] & 0xFFFFu);
-      b[t] = coop_get<BASE>(cell, w[t] >> 16);
-    }
-    if (u & (4u << 12)) {                  /* more than three products */
+    for (int t = 0; t < 6; ++t) acc = acc - a[t] * b[t];
+  } else {
 #pragma unroll
-      for (int t = 3; t < 6; ++t) {
-        a[t] = coop_get<SO_G>(cell, w[t] & 0xFFFFu);
-        b[t] = coop_get<BASE>(cell, w[t] >> 16);
-      }
-#pragma unroll
-      for (int t = 0; t < 6; ++t) acc = acc - a[t] * b[t];
-    } else {
-#pragma unroll
-      for (int t = 0; t < 3; ++t) acc = acc - a[t] * b[t];
-    }
+    for (int t = 0; t < 3; ++t) acc = acc - a[t] * b[t];
   }
   if (u & CL_END) {
     acc = coop_fold(acc, ctl, (u >> 9) & 7u);
 #if COOP_SPLIT
     if (PROG == P_LU) {
-      if (u & CL_DIAGS) {                  /* some lane ends a diagonal */
-        if ((ctl & (CL_LEAD | CL_DIAG)) == (CL_LEAD | CL_DIAG)) coop_put<SO_R>(cell, qa.x >> 16, 1.0 / acc);
-      }
-      if (!(ctl & CL_DIAG)) acc = acc * r;
-    } else {
-      acc = acc * r;
+      const double r = coop_get<L::G>(cell, e);   /* -1/U, or -1 */
+      if ((u & CL_DIAGS) && (ctl & (CL_LEAD | CL_DIAG)) == (CL_LEAD | CL_DIAG))
+        coop_put<L::G>(cell, e, -1.0 / acc);
+      if (!(ctl & CL_DIAG)) acc = -(acc * r);
     }
 #else
-    if ((ctl & (CL_LEAD | CL_SCALED)) == (CL_LEAD | CL_SCALED))
-      acc = acc / coop_get<SO_G>(cell, coop_diag[qa.x >> 19] & ~1);
+    if ((ctl & (CL_LEAD | CL_SCALED)) == (CL_LEAD | CL_SCALED)) acc = acc / coop_get<L::G>(cell, e);
 #endif
     coop_put_if<BASE>(ctl & CL_LEAD, cell, d, acc);
   }
@@ -381,16 +385,18 @@ __device__ __forceinline__ void coop_run(unsigned int cell, CoopFetch& f, int se
 #pragma unroll
     for (int d = 0; d < COOP_DEPTH; ++d) {
       const uint4 a = f.q[d][0], b = f.q[d][1];
-      if (PROG == P_RATE) {
-        coop_rate_op(cell, a, b, j, NT, n);
+      if (PROG == P_RATE || PROG == P_BUFD) {
+        coop_rate_op<NT, PROG == P_RATE ? CoopAt<NT>::A : CoopAt<NT>::B>(cell, a, b, j, NT, n);
         j += 4 * NT;
+      } else if (PROG == P_ONE || PROG == P_BUFP) {
+        coop_one_op<NT, PROG == P_ONE ? CoopAt<NT>::G : CoopAt<NT>::B>(cell, coef, a, b);
       } else if (PROG == P_DEST) {
-        acc = coop_dest_op(cell, acc, a, b);
+        acc = coop_dest_op<NT>(cell, acc, a, b);
       } else if (PROG == P_LU || PROG == P_SWEEP) {
         acc = coop_level_op<PROG, NT, NG>(cell, acc, a, b);
       } else {
-        acc = coop_sum_half<PROG>(cell, coef, acc, a);
-        acc = coop_sum_half<PROG>(cell, coef, acc, b);
+        acc = coop_sum_half<PROG, NT>(cell, coef, acc, a);
+        acc = coop_sum_half<PROG, NT>(cell, coef, acc, b);
       }
       /* into the registers just read: a load into others would be copied at
          the end of the loop, and the copy would wait for it */
@@ -400,12 +406,101 @@ __device__ __forceinline__ void coop_run(unsigned int cell, CoopFetch& f, int se
   }
 }
 
+/* Fun's long sums (a lane per sum, chains[32] = species, first product, blocks):
+   the products wait in B, so a term costs a load and an addition, in order. */
+template <int NT>
+__device__ __forceinline__ double coop_chain(const double* sm, int first, int blocks) {
+  const double2* b = reinterpret_cast<const double2*>(sm + CoopAt<NT>::B + first);
+  double s = 0.0;
+  const int most = __reduce_max_sync(0xFFFFFFFFu, blocks), last = blocks > 0 ? blocks - 1 : 0;
+  double2 v[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) v[t] = b[t];
+#pragma unroll 2
+  for (int k = 0; k < most; ++k) {
+    /* the next block's loads run during this one's additions */
+    const double2* nb = b + 4 * (k < last ? k + 1 : last);
+    double2 u[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) u[t] = nb[t];
+    double x = s;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) x = (x + v[t].x) + v[t].y;
+    s = k < blocks ? x : s;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = u[t];
+  }
+  return s;
+}
+
+#if COOP_TAIL
+/* The tail block's Schur complement becomes its negative inverse: Gauss-Jordan
+   elimination in place without pivoting (the factorisation has none), rows over
+   the warps, columns over the lanes.  A step scales the pivot row in its warp,
+   hands it over through A (free here; two rows in turn, so that one barrier per
+   step is enough) and updates the other rows, their factors coming from the
+   pivot column's lane.  ~250 cycles a step; the 62-level program that walked
+   these pivots took 49 of its levels, ~1,000 cycles each, for them. */
+template <int NT, int NG>
+__device__ __forceinline__ void coop_tail(double* sm) {
+  using L = CoopAt<NT>;
+  constexpr int M = COOP_TAIL, W = NT / 32, R = M / W, C = M / 32;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x % NT) >> 5;
+  double* D = sm + L::G + COOP_BLOCK;
+  double* buf = sm + L::A;
+  double a[R][C];
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+#pragma unroll
+    for (int c = 0; c < C; ++c) a[q][c] = D[(warp * R + q) * M + c * 32 + lane];
+#pragma unroll 1
+  for (int w = 0; w < W; ++w) {
+    const int kc = w * R / 32;                /* the pivots' column block */
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kl = (w * R + r) & 31;
+      double row[C];
+      if (warp == w) {
+        const double piv = __shfl_sync(0xFFFFFFFFu, C == 1 || kc == 0 ? a[r][0] : a[r][C - 1], kl);
+        const double inv = 1.0 / piv;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          row[c] = lane == kl && c == kc ? inv : a[r][c] * inv;
+          a[r][c] = row[c];
+          buf[(r & 1) * M + c * 32 + lane] = row[c];
+        }
+      }
+      coop_sync<NT, NG>();
+      if (warp != w) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) row[c] = buf[(r & 1) * M + c * 32 + lane];
+      }
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        if (q != r || warp != w) {
+          const double f = __shfl_sync(0xFFFFFFFFu, C == 1 || kc == 0 ? a[q][0] : a[q][C - 1], kl);
+#pragma unroll
+          for (int c = 0; c < C; ++c)
+            a[q][c] = (lane == kl && c == kc ? 0.0 : a[q][c]) - f * row[c];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+#pragma unroll
+    for (int c = 0; c < C; ++c) D[(warp * R + q) * M + c * 32 + lane] = -a[q][c];
+  coop_sync<NT, NG>();
+}
+#endif
+
 /* load the cell's column and set the integrator state (lane_start of the
    one-thread-per-cell kernels); attempt 1 is the retry: Hstart taken as 0
    and the retry tolerances */
 template <int NT, int NG>
 __device__ __forceinline__ void coop_start(CoopCell& c, const CoopArgs& a, double* sm, double* y,
                                            long col, int attempt) {
+  using L = CoopAt<NT>;
   const int tid = threadIdx.x % NT;
   c.col = col;
   c.attempt = attempt;
@@ -413,11 +508,11 @@ __device__ __forceinline__ void coop_start(CoopCell& c, const CoopArgs& a, doubl
   const double* rr = a.RCONST + col * NREACT;
 #pragma unroll
   for (int m = 0; m < (NVAR + NT - 1) / NT; ++m) y[m] = tid + m * NT < NVAR ? cc[tid + m * NT] : 0.0;
-  for (int i = NVAR + tid; i < COOP_NX; i += NT) sm[SO_V + i] = i < NSPEC ? cc[i] : coop_ext[i - NSPEC];
-  for (int j = tid; j < NREACT; j += NT) sm[SO_RX + j] = rr[j];
+  for (int i = NVAR + tid; i < COOP_NX; i += NT) sm[L::V + i] = i < NSPEC ? cc[i] : coop_ext[i - NSPEC];
+  for (int j = tid; j < NREACT; j += NT) sm[L::RX + j] = rr[j];
   for (int i = tid; i < COOP_NEXTRA; i += NT) {
     const int j = coop_extra_src[i];
-    sm[SO_RX + NREACT + i] = j >= 0 ? rr[j] * coop_extra_val[i] : coop_extra_val[i];
+    sm[L::RX + NREACT + i] = j >= 0 ? rr[j] * coop_extra_val[i] : coop_extra_val[i];
   }
   c.o = decode_options(a.ICNTRL + col * 20, a.RCNTRL + col * 20, a.tstart, a.tend, attempt);
   c.st.nfun = c.st.njac = c.st.nstp = c.st.nacc = 0;
@@ -500,13 +595,14 @@ __device__ __forceinline__ double coop_root(double x) {
    step_prologue, step_factor and step_stages in rodas3_kernels.cu. */
 template <int NT, int NG>
 __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, CoopFetch& f,
-                                            unsigned int cell, double* sm, double* y) {
+                                            unsigned int cell, double* sm, double* y, const int* place) {
+  using L = CoopAt<NT>;
   const int tid = threadIdx.x % NT;
   constexpr int NE = (NVAR + NT - 1) / NT;      /* species of a thread */
   const double Tend = a.tend;
   const double dir = (Tend >= a.tstart) ? 1.0 : -1.0;
-  double* s_err = sm + SO_RED;
-  int* s_ising = reinterpret_cast<int*>(sm + SO_RED + 8);
+  double* s_err = sm + L::RED;
+  int* s_ising = reinterpret_cast<int*>(sm + L::RED + 8);
 
   if (c.newstep) {
     /* TimeLoop exit tests and the H clamp */
@@ -545,21 +641,44 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
         if (s == -1) yn[m] = y[m];
         else if (s == 2) yn[m] = (y[m] + 2.0 * k1[m]) + 0.0 * k2[m];
         else yn[m] = yn[m] + 1.0 * k3[m];
-        if (k < NVAR) sm[SO_V + k] = yn[m];
+        if (k < NVAR) sm[L::V + k] = yn[m];
       }
       if (s >= 2) c.st.nfun += 1;
       coop_sync<NT, NG>();
       /* Fun_SPLIT: X = P_VAR - D_VAR*V; the destruction sums need no rates,
          so they run before the barrier that publishes A */
+      const int after = s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP;
       coop_run<P_RATE, NT, NG>(cell, f, COOP_SEG_RATE, COOP_SEG_DEST, NREACT);
+#if COOP_BUFFER
+      coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_BUFD);
+      coop_run<P_BUFD, NT, NG>(cell, f, COOP_SEG_BUFD, COOP_SEG_PROD, COOP_NBUFD);
+      coop_sync<NT, NG>();
+      /* the last warp adds up the long destruction sums, then the first the
+         long production sums, which wait for all products */
+      const int lane = tid & 31;
+      if (tid >= NT - 32) {
+        const int i = __ldg(coop_chain_of + 3 * lane);
+        const double d = coop_chain<NT>(sm, __ldg(coop_chain_of + 3 * lane + 1), __ldg(coop_chain_of + 3 * lane + 2));
+        if (i >= 0) sm[L::X + i] = d;
+      }
+      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, COOP_SEG_BUFP);
+      coop_run<P_BUFP, NT, NG>(cell, f, COOP_SEG_BUFP, after);
+      coop_sync<NT, NG>();
+      if (tid < 32) {
+        const int i = __ldg(coop_chain_of + 96 + 3 * lane);
+        const double p = coop_chain<NT>(sm, __ldg(coop_chain_of + 97 + 3 * lane), __ldg(coop_chain_of + 98 + 3 * lane));
+        if (i >= 0) sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i];
+      }
+#else
       coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_PROD);
       coop_sync<NT, NG>();
-      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
+      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, after);
+#endif
       coop_sync<NT, NG>();
     }
     if (s == -1) {
 #pragma unroll
-      for (int m = 0; m < NE; ++m) f0[m] = tid + m * NT < NVAR ? sm[SO_X + tid + m * NT] : 0.0;
+      for (int m = 0; m < NE; ++m) f0[m] = tid + m * NT < NVAR ? sm[L::X + tid + m * NT] : 0.0;
       /* Jac_SP straight into ros_PrepareMatrix's form: G = -JVS, a part of
          the columns at a time, then ghinv on the diagonal.  KppDecomp's
          singularity test reads each prepared diagonal before its row is
@@ -567,10 +686,11 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
          row + 1.  Diagonals without updates are final: their reciprocals. */
 #pragma unroll 1
       for (int q = 0; q < COOP_PARTS; ++q) {
-        const int seg = COOP_SEG_BPART0 + 2 * q;
+        const int seg = COOP_SEG_BPART0 + 3 * q;
         coop_run<P_RATE, NT, NG>(cell, f, seg, seg + 1, COOP_NBP(q));
         coop_sync<NT, NG>();
-        coop_run<P_JVS, NT, NG>(cell, f, seg + 1, q + 1 < COOP_PARTS ? seg + 2 : COOP_SEG_LU);
+        coop_run<P_JVS, NT, NG>(cell, f, seg + 1, seg + 2);
+        coop_run<P_ONE, NT, NG>(cell, f, seg + 2, q + 1 < COOP_PARTS ? seg + 3 : COOP_SEG_LU);
         coop_sync<NT, NG>();
       }
 #pragma unroll
@@ -578,11 +698,11 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
         const int k = tid + m * NT;
         if (k < NVAR) {
           const int o = __ldg(coop_diag + k);
-          const double g = coop_get<SO_G>(cell, o & ~1) + ghinv;
+          const double g = sm[L::G + (o >> 1)] + ghinv;
           if (fabs(g) < DBL_MIN) atomicMin(s_ising, k + 1);
-          coop_put<SO_G>(cell, o & ~1, g);
+          sm[L::G + (o >> 1)] = g;
 #if COOP_SPLIT
-          if (o & 1) sm[SO_R + k] = 1.0 / g;
+          if (o & 1) sm[L::G + L::RECIP + k] = -1.0 / g;
 #endif
         }
       }
@@ -599,6 +719,9 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
       }
       /* KppDecomp entry by entry, in levels */
       coop_run<P_LU, NT, NG>(cell, f, COOP_SEG_LU, COOP_SEG_SWEEP);
+#if COOP_TAIL
+      coop_tail<NT, NG>(sm);
+#endif
       continue;
     }
 #pragma unroll
@@ -616,10 +739,10 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
             v = v + (s == 0 ? dH * 0.5 : dH * 1.5) * dfdt;
           }
         } else {
-          v = (sm[SO_X + k] + hc1 * k1[m]) + hc2 * k2[m];
+          v = (sm[L::X + k] + hc1 * k1[m]) + hc2 * k2[m];
           if (s == 3) v = v + hc3 * k3[m];
         }
-        sm[SO_X + k] = v;
+        sm[L::X + k] = v;
       }
     }
     coop_sync<NT, NG>();
@@ -628,7 +751,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
     if (s < 3) {
 #pragma unroll
       for (int m = 0; m < NE; ++m) {
-        const double v = tid + m * NT < NVAR ? sm[SO_X + tid + m * NT] : 0.0;
+        const double v = sm[L::X + place[m]];
         if (s == 0) k1[m] = v;
         else if (s == 1) k2[m] = v;
         else k3[m] = v;
@@ -647,7 +770,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
     const int i = tid + m * NT;
     if (i < NVAR) {
       const double yi = y[m];
-      const double k4 = sm[SO_X + i];
+      const double k4 = sm[L::X + place[m]];
       yn[m] = (((yi + 2.0 * k1[m]) + 0.0 * k2[m]) + 1.0 * k3[m]) + 1.0 * k4;
       const double ye = (((0.0 + 0.0 * k1[m]) + 0.0 * k2[m]) + 0.0 * k3[m]) + 1.0 * k4;
       const double ymax = fmaxF(fabs(yi), fabs(yn[m]));
@@ -657,7 +780,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
 #if COOP_SPLIT
       err = err + q * q;
 #else
-      sm[SO_X + i] = q;
+      sm[L::X + i] = q;
 #endif
     }
   }
@@ -673,7 +796,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
   coop_sync<NT, NG>();
   if (tid == 0) {
     for (int i = 0; i < NVAR; ++i) {
-      const double q = sm[SO_X + i];
+      const double q = sm[L::X + i];
       err = err + q * q;
     }
     s_err[0] = err;
@@ -728,22 +851,28 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
    same stream words at about the same time and share them through L1; in
    between each synchronises on its own barrier. */
 template <int NT, int NG>
-__global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 256 / NT) rodas3_coop(CoopArgs a) {
+__global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 2) rodas3_coop(CoopArgs a) {
   __shared__ unsigned int s_pos[NG];
   const int g = NG == 1 ? 0 : threadIdx.x / NT, tid = threadIdx.x % NT;
-  double* sm = reinterpret_cast<double*>(coop_smem) + COOP_NCOEF + g * SO_CELL;
+  double* sm = reinterpret_cast<double*>(coop_smem) + COOP_NCOEF + g * CoopAt<NT>::CELL;
   const unsigned int cell = (unsigned int)__cvta_generic_to_shared(sm);
   for (int i = threadIdx.x; i < COOP_NCOEF; i += NT * NG)
     reinterpret_cast<double*>(coop_smem)[i] = coop_coef[i];
   if (tid == 0) {
-    sm[SO_G + NNZ] = sm[SO_X + NVAR] = sm[SO_A + NREACT] = sm[SO_RX + NREACT + COOP_NEXTRA] = 0.0;
-    sm[SO_R + NVAR] = 1.0;
+    using L = CoopAt<NT>;
+    sm[L::G + L::ZERO] = sm[L::X + NVAR] = sm[L::A + NREACT] = sm[L::RX + NREACT + COOP_NEXTRA] = 0.0;
+    sm[L::G + L::ZERO - 1] = -1.0;
   }
   __syncthreads();
   CoopFetch f;
   coop_prime<NT, NG>(f, COOP_SEG_RATE);
   CoopCell c;
-  double y[(NVAR + NT - 1) / NT];
+  constexpr int NE = (NVAR + NT - 1) / NT;
+  double y[NE];
+  int place[NE];              /* where the sweeps leave the thread's species */
+#pragma unroll
+  for (int m = 0; m < NE; ++m)
+    place[m] = tid + m * NT < NVAR ? (NT == 128 ? coop_place4 : coop_place8)[tid + m * NT] : NVAR;
   int have = 0, drained = 0;
   for (;;) {
     while (!have && !drained) {
@@ -763,22 +892,25 @@ __global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 256 / NT) rodas3_coop(Co
     } else if (!have) {
       break;
     }
-    if (have && coop_attempt<NT, NG>(c, a, f, cell, sm, y)) {
+    if (have && coop_attempt<NT, NG>(c, a, f, cell, sm, y, place)) {
       have = !coop_end<NT, NG>(c, a, sm, y);
       coop_sync<NT, NG>();    /* the result is stored before the next cell loads */
     }
   }
 }
 
-/* cells per block of the shared form */
-#define COOP_NG 3
+static size_t coop_smem_bytes(int threads, int cells) {
+  const int cell = threads == 128 ? CoopAt<128>::CELL : CoopAt<256>::CELL;
+  return ((size_t)cells * cell + COOP_NCOEF) * sizeof(double);
+}
 
-static size_t coop_smem_bytes(int cells) { return ((size_t)cells * SO_CELL + COOP_NCOEF) * sizeof(double); }
+/* cells per block of the shared form */
+#define COOP_NG 2
 
 /* the kernel instances: threads per cell (128 or 256), cells per block */
 static const void* coop_kernel(int threads, int cells) {
   if (threads == 128) return cells == 1 ? (const void*)rodas3_coop<128, 1> : (const void*)rodas3_coop<128, COOP_NG>;
-  if (threads == 256) return (const void*)rodas3_coop<256, 1>;
+  if (threads == 256) return cells == 1 ? (const void*)rodas3_coop<256, 1> : (const void*)rodas3_coop<256, COOP_NG>;
   return nullptr;
 }
 
@@ -786,27 +918,25 @@ static cudaError_t coop_attr(int threads, int cells) {
   const void* k = coop_kernel(threads, cells);
   if (!k) return cudaErrorInvalidValue;
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)coop_smem_bytes(cells));
+                              (int)coop_smem_bytes(threads, cells));
 }
 
 extern "C" int rodas3_coop_ok(void) {
-  return coop_smem_bytes(1) <= 227 * 1024 ? 1 : 0;
+  return coop_smem_bytes(128, 1) <= 227 * 1024 && coop_smem_bytes(256, 1) <= 227 * 1024 ? 1 : 0;
 }
 
-extern "C" size_t rodas3_coop_smem_bytes(void) { return coop_smem_bytes(1); }
+extern "C" size_t rodas3_coop_smem_bytes(void) { return coop_smem_bytes(128, 1); }
 
 extern "C" int rodas3_coop_blocks_per_sm(int threads) {
   if (!rodas3_coop_ok() || coop_attr(threads, 1) != cudaSuccess) return 0;
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, coop_kernel(threads, 1), threads,
-                                                    coop_smem_bytes(1)) != cudaSuccess)
+                                                    coop_smem_bytes(threads, 1)) != cudaSuccess)
     return 0;
   return nb;
 }
 
-/* bps: blocks per SM that the caller allows (0: as many as fit).  Up to two
-   cells per SM run in blocks of their own; larger batches put three in one
-   block, where they share the coefficients and the stream words. */
+/* bps: blocks per SM that the caller allows (0: as many as fit) */
 extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bps,
                                           cudaStream_t s) {
   if (!rodas3_coop_ok()) return cudaErrorInvalidValue;
@@ -814,7 +944,7 @@ extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bp
   const int occ = rodas3_coop_blocks_per_sm(threads);
   if (occ <= 0) return cudaErrorInvalidValue;
   int cells = 1, blocks = sms * (bps > 0 && bps < occ ? bps : occ);
-  if (threads == 128 && bps <= 0 && L->ncell > blocks && coop_smem_bytes(COOP_NG) <= 227 * 1024) {
+  if (bps <= 0 && L->ncell > blocks && coop_smem_bytes(threads, COOP_NG) <= 227 * 1024) {
     cells = COOP_NG;
     blocks = sms;
   }
@@ -830,13 +960,10 @@ extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bp
   a.qhead = L->qhead; a.nfail = L->nfail; a.ATOLr = L->ATOLr; a.RTOLr = L->RTOLr;
   a.ckpt = L->ckpt; a.ckpt_max = L->ckpt_max;
   cudaMemsetAsync(L->qhead, 0, sizeof(unsigned int), s);
-  const size_t smem = coop_smem_bytes(cells);
-  if (threads == 256)
-    rodas3_coop<256, 1><<<blocks, 256, smem, s>>>(a);
-  else if (cells == 1)
-    rodas3_coop<128, 1><<<blocks, 128, smem, s>>>(a);
-  else
-    rodas3_coop<128, COOP_NG><<<blocks, 128 * COOP_NG, smem, s>>>(a);
+  void* args[] = {&a};
+  const cudaError_t el = cudaLaunchKernel(coop_kernel(threads, cells), dim3(blocks), dim3(threads * cells),
+                                          args, coop_smem_bytes(threads, cells), s);
+  if (el != cudaSuccess) return el;
   return cudaGetLastError();
 }
 

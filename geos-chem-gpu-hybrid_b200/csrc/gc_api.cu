@@ -39,17 +39,21 @@ const int kMaxDev = 64;
 /* launch mode until set_launch or GCCHEM_B200_MODE names a kernel: chosen per
    call by the number of cells (auto_mode) */
 const int kAuto = -1;
-/* The cooperative kernel solves a cell in a twentieth of the time one thread
-   takes, but keeps only three cells per SM; one thread per cell catches up
-   once the batch fills the GPU several times.  Full cold steps on a B200,
-   cooperative / persistent: fullchem 1,000 cells 0.035 / 0.549 s, 16,000 cells
-   0.468 / 1.052 s, 40,000 cells 1.151 / 1.436 s; at 238,464 cells 2.9 M / 4.6 M
-   attempts per second.  Without the fused factorisation (synthetic mechanism)
-   the cooperative kernel wins at every size: 1,500 cells 0.034 / 0.692 s,
-   1.5 M / 0.8 M attempts per second at full load.  The --fmad=false build may
-   not split sums over lanes: 100 cells 0.108 / 0.553 s, even at about 1,000. */
+/* The cooperative kernel solves a cell in a thirtieth of the time one thread
+   takes, but keeps only two cells per SM; one thread per cell catches up once
+   the batch fills the GPU several times.  Full cold steps on a B200,
+   cooperative / persistent: fullchem 1 cell 0.009 / 0.262 s, 1,000 cells 0.030 /
+   0.549 s, 16,000 cells 0.47 / 1.05 s, 29,952 cells 0.88 / 1.25 s, 238,464
+   cells 2.9 M / 4.6 M attempts per second.  The line is drawn below the
+   crossover (about 50,000 cells): one cell in 10^5 has a step-size sequence that
+   amplifies any difference in rounding to 1e-8 and more, so that only batches
+   that gain at least twofold leave the arithmetic of the thread-per-cell
+   kernels.  Without the fused factorisation (synthetic mechanism) the
+   cooperative kernel wins at every size: 1,500 cells 0.022 / 0.66 s, 2.3 M /
+   0.8 M attempts per second at full load.  The --fmad=false build may not
+   split sums over lanes: 100 cells 0.14 / 0.56 s, even at about 1,000. */
 #if defined(GC_LU_RECIP) && GC_LU_RECIP
-const int kCoopCells = 64000;
+const int kCoopCells = 16000;
 const bool kCoopAlways = true;      /* without the fused factorisation */
 #else
 const int kCoopCells = 1000;

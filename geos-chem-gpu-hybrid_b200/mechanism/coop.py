@@ -231,34 +231,72 @@ def compile_tables(mech: dict):
 # the warp executes them.  The addresses of a stream are known in advance, so
 # the kernel fetches operations several ahead of their use.
 #
-# Operands are given as byte offsets in their array (the kernel keeps the cell
-# in shared memory), so that a word needs no arithmetic; a missing operand
-# points at a constant 0 (or 1) behind the array, so that it needs no test.
+# Rates and sums give operands as byte offsets in their array (the kernel keeps
+# the cell in shared memory), level operations as element indices; a missing
+# operand is the index of a constant 0 (or 1) behind the array, so that it
+# needs no test.
 #
 #   rate operations   four products (f0 | f1<<16, f2 | f3<<16).  Product k of
 #                     operation i of warp w and lane l is number
 #                     ((i*4 + k)*NW + w)*32 + l.
 #   dest operations   header, control, three products (f0 | f1<<16, f2)
 #   sum operations    two halves of a header and three words (prod, jvs)
+#   single operations four pairs (entry | coefficient<<16, partial)
 #   level operations  header, control, six words (lu, sweep)
 #
 # Control word, per lane: L_* flags, log2 of the lane's group, exchanges that
-# the warp does (the largest of its groups), products in use, a chain's first
-# step, block barriers after the operation.  A sum's header is its entry's
-# offset | control << 16; a level's is the entry's offset | the offset of its
-# scale in R << 16.
+# the warp does (the largest of its groups), products in use, block barriers
+# after the operation.  A sum's header is its entry's offset | control << 16; a
+# level's is the entry's index | the index of its scale << 16.
+#
+# The sweeps of the production build use partitioned inverses (Alvarado and
+# Schreiber, Optimal parallel solution of sparse triangular systems, 1993):
+# consecutive levels form a part whose rows get the entries of the inverse of
+# their diagonal block, so that a part is solved by one level (its rows'
+# products with the inverse) after one level that subtracts the terms outside
+# the part.  fullchem: 5 parts, 8 levels instead of 70.  The inverses are rows
+# of the same recurrence as the factors and are formed by the factorisation's
+# program, next to the entries that become final at the same level:
+#
+#   forward, unit diagonal   V(i,j) = L(i,j) - sum_c L(i,c) V(c,j),
+#                            x_i = b_i - sum_j V(i,j) b_j
+#   backward                 T(i,j) = (U(i,j) R_j - sum_c U(i,c) T(c,j)) R_i,
+#                            x_i = R_i b_i - sum_j T(i,j) b_j,   R = 1/U(i,i)
+#
+# with c over the row's columns inside the part.
+#
+# The last rows are nearly dense and their pivots follow one another, two
+# levels each (fullchem: 49 of the 62 levels belong to the last 32 rows).  They
+# are left out of the levels: the program only forms their Schur complement,
+# which one block-wide Gauss-Jordan elimination turns into its negative inverse,
+# rows over warps and columns over lanes; the sweeps then need one level for
+# these rows.
+#
+# The factor array of a cell is [G | tail block | V and T | -R | -1 | 0]; the
+# vector array is [X | 0 | Z], where a row's solution goes to the other half
+# when its part's rows are still read.
+#
+# The order of the terms of Fun's sums is the reference's in every build: the
+# difference of production and destruction is where their rounding is amplified
+# most (a step size of a sensitive cell moves by 1e-7 relative when these sums
+# are split over lanes, by 1e-8 when all the others are).  Long ones are formed
+# in two passes: all threads write their products one after the other into a
+# buffer, then one lane per sum adds them up, two instructions per term.
 
 WORDS = 8
 DEPTH = 4              # operations fetched ahead; a segment is a multiple of it
-L_LEAD, L_FIRST, L_END, L_CHAIN, L_DIAG, L_SCALED = 1, 2, 4, 8, 16, 32
-L_DIAGS = 1 << 15      # factorisation: some lane of the warp has L_DIAG
-L_GROUP, L_FOLD, L_USED, L_STEP, L_SYNC = 6, 9, 12, 15, 20
-CHAIN_MAX = 32         # rows of a warp chain (one lane per row)
+L_LEAD, L_FIRST, L_END, L_START, L_DIAG, L_SCALED = 1, 2, 4, 8, 16, 32
+L_DIAGS = 1 << 15      # some lane of the warp has L_DIAG
+L_GROUP, L_FOLD, L_USED, L_SYNC = 6, 9, 12, 20
 # cycles of an operation: fixed part, per product, per exchange, end of an
-# entry (measured latencies on a B200: shared memory 29, FP64 FMA 9, barrier of
-# 128 threads 19; a lone warp issues every ~3 cycles); they only steer how far
-# sums are split
-OP_COST, TERM_COST, FOLD_COST, END_COST = 70, 18, 40, 40
+# entry (an operation of six products and three exchanges measures ~650 on a
+# B200); they steer how far sums are split and which parts get inverses
+OP_COST, TERM_COST, FOLD_COST, END_COST = 250, 25, 45, 60
+
+
+BLOCK = 8              # terms that a chain adds between two tests of its length
+NO_ENTRY = 0xFFFF      # single operations: an idle pair
+LONG = 30              # terms of Fun's sums above which a sum goes through the buffer
 
 
 def _lanes(items, k, split):
@@ -344,8 +382,8 @@ class Segment:
                 if x < len(lanes):
                     (head, flags), lg, words = lanes[x]
                     w = words[per_op * t:per_op * (t + 1)]
-                    lead = 0 if x % (1 << lg) else L_LEAD
-                    out.append((head, ctl | lead | flags | lg << L_GROUP, w + [self.none] * (per_op - len(w))))
+                    lead = flags & ~L_START if x % (1 << lg) else flags | L_LEAD
+                    out.append((head, ctl | lead | lg << L_GROUP, w + [self.none] * (per_op - len(w))))
                 else:
                     out.append((self.head, ctl, [self.none] * per_op))
             yield out
@@ -370,6 +408,16 @@ class Segment:
                                     for (h, c, w), (g, d, u) in zip(a, b)])
         return self.pad([self.head] + [self.none] * 3 + [self.head] + [self.none] * 3)
 
+    def singles(self, items):
+        """Entries of one product: four (entry | coefficient<<16, partial)
+        pairs per lane."""
+        for n, (head, word) in enumerate(items):
+            v, w = n // 32 % self.nw, n // (32 * self.nw)
+            if w % 4 == 0 and len(self.ops[v]) == w // 4:
+                self.ops[v].append([self.idle() for _ in range(32)])
+            self.ops[v][w // 4][n % 32][w % 4 * 2:w % 4 * 2 + 2] = [head | (word & 0xFFFF) << 16, word >> 16]
+        return self.pad()
+
     def level(self, items, split):
         warps, cost = _place(items, self.nw, split, 6)
         self.cost += cost + 30
@@ -378,25 +426,6 @@ class Segment:
                 diags = L_DIAGS if any(flags & L_DIAG for (_, flags), _, _ in lanes) else 0
                 for op in self._split(lanes, 6):
                     self.ops[v].append([[h, c | diags] + w for h, c, w in op])
-        self._sync()
-
-    def chain(self, rows, pos):
-        """A warp chain over `rows` [(header, flags)]: lane r owns row r; step
-        j broadcasts row j's value and every lane with an entry (r, j)
-        subtracts its term."""
-        m = len(rows)
-        for j0 in range(0, m, 6):
-            used = min(6, m - j0)
-            ctl = (L_FIRST if j0 == 0 else 0) | (L_END if j0 + used == m else 0) | \
-                used << L_USED | L_CHAIN | j0 << L_STEP
-            op = []
-            for r in range(32):
-                head, flags, lead = rows[r] + (L_LEAD,) if r < m else (self.head, rows[0][1], 0)
-                op.append([head, ctl | lead | flags] +
-                          [pos.get((r, j), self.none & 0xFFFF) if j < m else self.none & 0xFFFF
-                           for j in range(j0, j0 + 6)])
-            self.ops[0].append(op)
-        self.cost += 45 * m + 100
         self._sync()
 
     def _sync(self):
@@ -408,47 +437,37 @@ class Segment:
                 lane[1] += 1 << L_SYNC
 
 
-def _sweep(seg, n, deps, split, forward):
-    """Levels of a triangular sweep.  deps[i]: [(column, factor position)] in
-    the reference's order.  Runs of levels with very few rows become warp
-    chains (at most CHAIN_MAX rows): first one level subtracts every term whose
-    column lies outside the chain, then one warp walks the chain."""
-    one = 8 * n << 16                    # offset of the constant 1 behind R
-
-    def head(i):
-        return (8 * i | one, 0) if forward else (8 * i | 8 * i << 16, L_SCALED)
-
+def _sweep_levels(n, deps, order):
     lev = [0] * n
-    order = list(range(n)) if forward else list(range(n - 1, -1, -1))
     for i in order:
-        lev[i] = max([lev[c] + 1 for c, _ in deps[i]] + [0])
+        lev[i] = max([lev[c] + 1 for c, _ in deps[i] if c < n] + [0])
+    return lev
+
+
+def _parts(n, deps, order, limit):
+    """Parts of a triangular sweep: runs of levels whose diagonal block's
+    inverse has at most `limit` entries more than the block.  Returns [(rows in
+    order, {row: columns of its inverse inside the part})]."""
+    lev = _sweep_levels(n, deps, order)
     nlev = max(lev) + 1 if n else 0
-    by = [[i for i in order if lev[i] == k] for k in range(nlev)]
 
-    def items(rows, skip=(), bulk=False):
-        return [((8 * i | one, 0) if bulk else head(i), [8 * p | 8 * c << 16 for c, p in deps[i] if c not in skip])
-                for i in rows]
+    def part(k, e):
+        rows = sorted((i for i in order if k <= lev[i] < e), key=lambda i: lev[i])
+        inside, reach, fill = set(rows), {}, 0
+        for i in rows:
+            cols = [c for c, _ in deps[i] if c in inside]
+            reach[i] = set(cols).union(*[reach[c] for c in cols])
+            fill += len(reach[i]) - len(cols)
+        return rows, reach, fill
 
-    k = 1 if forward else 0              # the forward sweep leaves level 0 as it is
+    out, k = [], 0
     while k < nlev:
-        e = k
-        if split:
-            rows = 0
-            while e < nlev and len(by[e]) <= (4 if e == 0 else 2) and rows + len(by[e]) <= CHAIN_MAX:
-                rows += len(by[e])
-                e += 1
-        if e - k >= 4:
-            rows = [i for q in range(k, e) for i in by[q]]
-            inside = {i: r for r, i in enumerate(rows)}
-            bulk = [it for it in items(rows, inside, True) if it[1]]
-            if bulk:
-                seg.level(bulk, split)
-            seg.chain([head(i) for i in rows],
-                      {(inside[i], inside[c]): 8 * p for i in rows for c, p in deps[i] if c in inside})
-            k = e
-        else:
-            seg.level(items(by[k]), split)
-            k += 1
+        e = k + 1
+        while e < nlev and part(k, e + 1)[2] <= limit:
+            e += 1
+        out.append(part(k, e)[:2])
+        k = e
+    return out
 
 
 def level_programs(mech: dict, split: bool, nw: int):
@@ -459,7 +478,7 @@ def level_programs(mech: dict, split: bool, nw: int):
         return None
     n, nfix, nnz, nreact = mech["nvar"], mech["nfix"], mech["nnz"], mech["nreact"]
     crow, diag, icol, where = mech["lu_crow"], mech["lu_diag"], mech["lu_icol"], mech["lu_where"]
-    if nnz >= (1 << 13) - 1:           # byte offsets of 16 bits
+    if 8 * nnz >= 1 << 16:             # byte offsets of 16 bits
         return None
     extra = {}                 # first factors behind the rate constants: (reaction or
                                # -1, literal), the literal itself or RCT(j)*literal
@@ -586,8 +605,36 @@ def level_programs(mech: dict, split: bool, nw: int):
 
     no_rate, no_dest, no_sum = (zero | one << 16, one | one << 16), (zero | one << 16, one), 8 * nreact << 16
     segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
-            "dest": Segment(nw, no_dest).dest([((8 * i, 0), [dword(f) for f in w]) for i, w in dest], split),
-            "prod": Segment(nw, no_sum).sums([((8 * i, 0), scaled_words(w)) for i, w in prod], split)}
+            "dest": None, "bufd": None, "prod": None, "bufp": None}
+    long_d = [i for i, w in dest if split and len(w) > LONG]
+    long_p = [i for i, w in prod if split and (len(w) > LONG or i in long_d)]
+    if len(long_p) > 32:
+        return None
+    # the buffer: the long sums' products, each sum padded to whole blocks
+    first = {}
+
+    def buffer(key, sums, none, at):
+        out = []
+        for i, words in sums:
+            first[(key, i)] = (at + len(out), -(-len(words) // BLOCK))
+            out += words + [none] * (-len(words) % BLOCK)
+        return out
+
+    rates_d = buffer("d", [(i, [words4(f) for f in w]) for i, w in dest if i in long_d], list(no_rate), 0)
+    ones_p = buffer("p", [(i, scaled_words(w)) for i, w in prod if i in long_p], no_sum, len(rates_d))
+    if not long_p:
+        del segs["bufd"], segs["bufp"]
+    segs["dest"] = Segment(nw, no_dest).dest([((8 * i, 0), [dword(f) for f in w])
+                                              for i, w in dest if i not in long_d], False)
+    if long_p:
+        segs["bufd"] = Segment(nw, no_rate, None).rates(rates_d)
+    segs["prod"] = Segment(nw, no_sum).sums([((8 * i, 0), scaled_words(w))
+                                             for i, w in prod if i not in long_p], False)
+    if long_p:
+        segs["bufp"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(
+            [(8 * (len(rates_d) + k), w) for k, w in enumerate(ones_p)])
+    # lane l's chain: species, first product, blocks
+    chains = [[(i,) + first[(key, i)] for i in rows] for key, rows in (("d", long_d), ("p", long_p))]
     # KppDecomp entry by entry: G(i,c) = G(i,c) - sum L(i,j) U(j,c), and for
     # c < i the product with 1/U(c,c); an entry's level is one above those of
     # the factors (and of the pivot) that it reads
@@ -598,37 +645,174 @@ def level_programs(mech: dict, split: bool, nw: int):
             j = icol[kk]
             for jj in range(diag[j] + 1, crow[j + 1]):
                 upd[where[(i, icol[jj])]].append((kk, jj))
+    # the tail block: its entries live in a dense array behind G
+    tail = _tail_rows(n, row_of, icol) if split else 0
+    t0 = n - tail
+    in_tail = [row_of[p] >= t0 and icol[p] >= t0 for p in range(nnz)]
+    block = nnz - sum(in_tail)
+    place = [0] * nnz                    # where an entry of the LU pattern lives
+    for k, p in enumerate(p for p in range(nnz) if not in_tail[p]):
+        place[p] = k
+    for p in range(nnz):
+        if in_tail[p]:
+            place[p] = block + (row_of[p] - t0) * tail + icol[p] - t0
+    if 2 * tail > nreact or 8 * (block + tail * tail) > NO_ENTRY:
+        return None
     # -Jac0 (the coefficients carry the sign); the kernel adds ghinv to the
     # diagonal and forms the reciprocals of the diagonals without updates
+    fill = set(range(block, block + tail * tail)) - {place[p] for p in range(nnz)}
     for q, part in enumerate(bpart):
+        mine = [(8 * place[p], scaled_words(jvs[p])) for p in range(nnz) if part_of[icol[p]] == q]
+        mine += [(8 * p, []) for p in sorted(fill)] if q == 0 else []
         segs[f"bpart{q}"] = Segment(nw, no_rate, None).rates([words4(f) for f in part])
-        segs[f"jvs{q}"] = Segment(nw, no_sum).sums(
-            [((8 * p, 0), scaled_words(jvs[p])) for p in range(nnz) if part_of[icol[p]] == q], split)
-    elev = [0] * nnz
-    for i in range(n):
-        for p in range(crow[i], crow[i + 1]):
-            c = icol[p]
-            lv = max([max(elev[a], elev[b]) + 1 for a, b in upd[p]] + [0])
-            if c < i:
-                lv = max(lv, elev[diag[c]] + 1)
-            elev[p] = lv
-    none = 8 * nnz | 8 * nnz << 16       # the constant 0 behind G, times itself
-    lu = segs["lu"] = Segment(nw, none, 8 * nnz | 8 * n << 16)
-    for k in range(1, max(elev) + 1):
-        items = []
-        for p in range(nnz):
-            if elev[p] == k:
-                i, c = row_of[p], icol[p]
-                head = (8 * p | 8 * (c if c <= i else n) << 16, L_SCALED if c < i else L_DIAG if c == i else 0)
-                items.append((head, [8 * a | 8 * b << 16 for a, b in upd[p]]))
-        lu.level(items, split)
-    sweep = segs["sweep"] = Segment(nw, 8 * nnz | 8 * n << 16, 8 * n | 8 * n << 16)
-    _sweep(sweep, n, [[(icol[p], p) for p in range(crow[i], diag[i])] for i in range(n)], split, True)
-    _sweep(sweep, n, [[(icol[p], p) for p in range(diag[i] + 1, crow[i + 1])] for i in range(n)], split, False)
-    lu.pad(), sweep.pad()
+        segs[f"jvs{q}"] = Segment(nw, no_sum).sums([((h, 0), w) for h, w in mine if len(w) > 1], split)
+        segs[f"one{q}"] = [(h, w[0] if w else no_sum) for h, w in mine if len(w) <= 1]
+    lower = [[(icol[p], place[p]) for p in range(crow[i], diag[i])] for i in range(n)]
+    upper = [[(icol[p], place[p]) for p in range(diag[i] + 1, crow[i + 1])] for i in range(n)]
+    # entries (row, column, place, updates by the pivots before the tail)
+    entries = [(row_of[p], icol[p], place[p], [(place[a], place[b]) for a, b in upd[p] if icol[a] < t0])
+               for p in range(nnz)]
+    at_diag = [place[p] for p in diag]
+    limits = None
+    if split:
+        tried = [(f, u) for f in INVERSE_LIMITS for u in INVERSE_LIMITS]
+        limits = min(tried, key=lambda lim: _factor_and_sweeps(
+            n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["cost"])
+    best = _factor_and_sweeps(n, tail, block, entries, at_diag, lower, upper, split, nw, limits)
+    for q in range(len(bpart)):
+        segs[f"one{q}"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(segs[f"one{q}"])
+    segs["lu"], segs["sweep"] = best["lu"], best["sweep"]
     return {"segs": segs, "parts": len(parts), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
-            "nbp": [len(part) for part in parts],
-            "diag": [(8 * diag[i], not upd[diag[i]]) for i in range(n)]}
+            "nbp": [len(part) for part in parts], "ng": best["ng"], "place": best["place"], "tail": tail,
+            "chains": chains, "buffer": len(rates_d) + len(ones_p), "nbufd": len(rates_d), "factor": place, "block": block, "diag": [(at_diag[i], i < t0 and not upd[diag[i]]) for i in range(n)],
+            "cost": best["cost"]}
+
+
+# most entries that a part's inverse may add; every pair is tried
+INVERSE_LIMITS = (0, 50, 100, 200, 400)
+
+
+def _tail_rows(n, row_of, icol):
+    """Rows of the tail block: 64 where they are dense, else 32."""
+    for m, least in ((64, 0.9), (32, 0.0)):
+        if n >= 2 * m - 8 and sum(r >= n - m and c >= n - m for r, c in zip(row_of, icol)) >= least * m * m:
+            return m
+    return 0
+
+
+def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, limits, estimate=False):
+    """The factorisation's program (with the inverses of the sweeps' parts) and
+    the sweeps' one, for one choice of parts; estimate: only their cost, the
+    factorisation's from the products per level."""
+    t0 = n - tail
+    fwd, bwd = ([], []) if limits is None else \
+        (_parts(t0, lower, range(t0), limits[0]), _parts(t0, upper, range(t0 - 1, -1, -1), limits[1]))
+    at = {}                                # (row, column) -> index of V or T
+    for parts in (fwd, bwd):
+        for rows, reach in parts:
+            for i in rows:
+                for j in sorted(reach[i]):
+                    at[(i, j)] = block + tail * tail + len(at)
+    rbase = block + tail * tail + len(at)    # -R, then -1, then 0
+    minus, zero = rbase + n, rbase + n + 1
+    # nodes: index, start value read, scale, flags, products
+    level, nodes = {minus: 0}, []
+
+    def node(index, start, scale, flags, terms):
+        lv = max([max(level[a], level[b]) + 1 for a, b in terms] + [0])
+        if scale != minus and not flags & L_DIAG:
+            lv = max(lv, level[scale] + 1)
+        level[index] = lv
+        if flags & L_DIAG:
+            level[scale] = lv
+        if lv:
+            nodes.append((lv, index, start, scale, flags, terms))
+
+    for i, c, p, terms in entries:
+        if c < i and c < t0:
+            node(p, True, rbase + c if split else diag[c], L_SCALED, terms)
+        elif c == i and i < t0:
+            node(p, True, rbase + c, L_DIAG, terms)
+        else:
+            node(p, True, minus, 0, terms)
+    for rows, reach in fwd:
+        for i in rows:
+            for j in sorted(reach[i]):
+                terms = [(p, minus) for c, p in lower[i] if c == j]
+                terms += [(p, at[(c, j)]) for c, p in lower[i] if c > j and (i, c) in at and (c, j) in at]
+                node(at[(i, j)], False, minus, 0, terms)
+    for rows, reach in bwd:
+        for i in rows:
+            for j in sorted(reach[i]):
+                terms = [(p, rbase + j) for c, p in upper[i] if c == j]
+                terms += [(p, at[(c, j)]) for c, p in upper[i] if c < j and (i, c) in at and (c, j) in at]
+                node(at[(i, j)], False, rbase + i, L_SCALED, terms)
+    lu = Segment(nw, zero | zero << 16, zero | minus << 16)
+    last = max(level.values())
+    if estimate:
+        work = [0] * (last + 1)
+        for lv, _, _, _, _, terms in nodes:
+            work[lv] += len(terms)
+        lu.cost = sum(400 + 70 * w // (32 * nw) for w in work)
+        nodes, last = [], 0
+    by = [[] for _ in range(last + 1)]
+    work = [0] * (last + 1)
+    late = []
+    for lv, index, start, scale, flags, terms in nodes:
+        early = [t for t in terms if max(level[t[0]], level[t[1]]) + 1 <= lv - EARLY] if split else []
+        if len(early) < 3:
+            early = []
+        rest = [t for t in terms if t not in early] if early else terms
+        by[lv].append((index, start or bool(early), scale, flags, rest))
+        work[lv] += len(rest)
+        if early:
+            late.append((max(max(level[a], level[b]) + 1 for a, b in early), lv, index, start, early))
+    # the bulk of a long sum runs at the emptiest level between its operands
+    # and its end, so that the end is short
+    for lo, hi, index, start, early in sorted(late, key=lambda x: -len(x[4])):
+        k = min(range(lo, hi), key=lambda q: (work[q], q))
+        by[k].append((index, start, minus, 0, early))
+        work[k] += len(early)
+    for k in range(1, last + 1):
+        lu.level([((index | scale << 16, flags | (L_START if start else 0)), [a | b << 16 for a, b in terms])
+                  for index, start, scale, flags, terms in by[k]], split)
+    sweep = Segment(nw, zero | n << 16, n | minus << 16)
+    x = list(range(n))                     # where a row's current value is
+    if limits is None:
+        for deps, order, scaled in ((lower, range(n), False), (upper, range(n - 1, -1, -1), True)):
+            lev = _sweep_levels(n, deps, order)
+            for k in range(0 if scaled else 1, max(lev) + 1):
+                sweep.level([((i | (diag[i] if scaled else minus) << 16, L_START | (L_SCALED if scaled else 0)),
+                              [p | c << 16 for c, p in deps[i]]) for i in order if lev[i] == k], split)
+    for parts, deps, scaled in ((fwd, lower, False), (bwd, upper, True)):
+        for rows, reach in parts:
+            inside = set(rows)
+            out = [(i, [p | x[c] << 16 for c, p in deps[i] if c not in inside]) for i in rows]
+            out = [((x[i] | minus << 16, L_START), w) for i, w in out if w]
+            if out:
+                sweep.level(out, split)
+            new, items = list(x), []
+            for i in rows:
+                if scaled or reach[i]:
+                    new[i] = (x[i] + n + 1) % (2 * n + 2)
+                    items.append(((new[i] | minus << 16, 0), [(rbase + i if scaled else minus) | x[i] << 16] +
+                                  [at[(i, j)] | x[j] << 16 for j in sorted(reach[i])]))
+            if items:
+                sweep.level(items, split)
+            x = new
+        if tail and not scaled:            # the tail block, once both sweeps reach it
+            out = [(i, [p | x[c] << 16 for c, p in lower[i] if c < t0]) for i in range(t0, n)]
+            sweep.level([((x[i] | minus << 16, L_START), w) for i, w in out if w], split)
+            new = [i if i < t0 else i + n + 1 for i in range(n)]
+            sweep.level([((new[i] | minus << 16, 0),
+                          [block + (i - t0) * tail + j - t0 | x[j] << 16 for j in range(t0, n)])
+                         for i in range(t0, n)], split)
+            x = x[:t0] + new[t0:]
+    lu.pad(), sweep.pad()
+    return {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
+
+
+EARLY = 2              # levels between an early product's readiness and its sum's end
 
 
 def coop_inc(mech: dict) -> str:
@@ -656,15 +840,19 @@ def coop_inc(mech: dict) -> str:
             if nw == 4:
                 lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
                           f"#define COOP_NEXTRA {len(p['extra'])}", f"#define COOP_PARTS {p['parts']}",
-                          "#define COOP_NSEG %d" % len(p["segs"]),
                           doubles("coop_ext", p["ext"]),
                           arr("int", "coop_extra_src", [j for j, _ in p["extra"]]),
                           doubles("coop_extra_val", [v for _, v in p["extra"]]),
-                          f"#define COOP_NCOEF {len(p['coef'])}", doubles("coop_coef", p["coef"]),
-                          "#define COOP_NBP(q) (%s)" % " : ".join(
+                          f"#define COOP_NCOEF {len(p['coef']) + len(p['coef']) % 2}",
+                          doubles("coop_coef", list(p["coef"]) + [0.0] * (len(p["coef"]) % 2)),
+                          f"#define COOP_BUFFER {p['buffer']}", f"#define COOP_NBUFD {p['nbufd']}",
+                          arr("int", "coop_chain_of", [x for c in p["chains"] for k in range(32)
+                                                    for x in (c[k] if k < len(c) else (-1, 0, 0))]),
+                          f"#define COOP_TAIL {p['tail']}", f"#define COOP_BLOCK {p['block']}", "#define COOP_NBP(q) (%s)" % " : ".join(
                               [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),
-                          arr("int", "coop_diag", [o | (e and 1) for o, e in p["diag"]])]
+                          arr("int", "coop_diag", [o << 1 | (e and 1) for o, e in p["diag"]])]
                 lines += [f"#define COOP_SEG_{name.upper()} {k}" for k, name in enumerate(p["segs"])]
+            lines += [f"#define COOP_NG{nw} {p['ng']}", arr("int", f"coop_place{nw}", p["place"])]
             words, where = [], []
             for seg in p["segs"].values():
                 for ops in seg.ops:

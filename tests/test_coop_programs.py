@@ -11,6 +11,7 @@ of differently ordered sums.
 """
 import numpy as np
 import pytest
+from scipy.linalg import solve_triangular
 
 from mechanism import codegen, coop
 
@@ -28,18 +29,19 @@ def case(request):
 
 
 class Array:
-    """Elements addressed by byte offset; the one behind the last is a constant."""
+    """Elements addressed by byte offset (unit 8) or index (unit 1); the one
+    behind the last may not be written."""
 
-    def __init__(self, values, last):
-        self.v = list(values) + [last]
+    def __init__(self, values, last, unit=8):
+        self.v, self.unit = list(values) + [last], unit
 
     def __getitem__(self, off):
-        assert off % 8 == 0
-        return self.v[off // 8]
+        assert off % self.unit == 0
+        return self.v[off // self.unit]
 
     def __setitem__(self, off, x):
-        assert off % 8 == 0 and off // 8 < len(self.v) - 1
-        self.v[off // 8] = x
+        assert off % self.unit == 0 and off // self.unit < len(self.v) - 1
+        self.v[off // self.unit] = x
 
 
 def _rates(seg, product, n):
@@ -86,11 +88,11 @@ def _sums(seg, kind, product, finish):
             continue
         ctl = [c for _, c, _ in step]
         assert len({c & (coop.L_FIRST | coop.L_END) for c in ctl}) == 1
+        if ctl[0] & coop.L_FIRST:
+            acc = [0.0] * 32
         for x, (_, c, words) in enumerate(step):
-            a = 0.0 if c & coop.L_FIRST else acc[x]
             for w in words:
-                a = product(a, w)
-            acc[x] = a
+                acc[x] = product(acc[x], w)
         if ctl[0] & coop.L_END:
             acc = _fold(acc, ctl)
             for x, (h, c, _) in enumerate(step):
@@ -98,7 +100,7 @@ def _sums(seg, kind, product, finish):
                     finish(h, acc[x])
 
 
-def _levels(seg, start, product, scale, finish):
+def _levels(seg, G, X, finish):
     """All warps from barrier to barrier; finished entries become visible at
     the next one.  Every warp must pass the same number of barriers."""
     place, wait = [(0, [0.0] * 32)] * seg.nw, [0] * seg.nw
@@ -114,44 +116,26 @@ def _levels(seg, start, product, scale, finish):
                 op = ops[i]
                 i += 1
                 ctl = [x[1] for x in op]
-                uniform = coop.L_FIRST | coop.L_END | coop.L_CHAIN | -1 << coop.L_FOLD
+                uniform = coop.L_FIRST | coop.L_END | -1 << coop.L_FOLD
                 assert len({c & uniform for c in ctl}) == 1
                 if ctl[0] & coop.L_FIRST:
-                    acc = [start(x[0] & 0xFFFF) if x[1] & coop.L_LEAD else 0.0 for x in op]
+                    acc = [X[x[0] & 0xFFFF] if x[1] & coop.L_START else 0.0 for x in op]
                 used = (ctl[0] >> coop.L_USED) & 7
-                if ctl[0] & coop.L_CHAIN:
-                    for t in range(used):
-                        j = ((ctl[0] >> coop.L_STEP) & 31) + t
-                        xj = scale(op[j][0] >> 16, op[j][1], acc[j])
-                        for x in range(32):
-                            if op[x][2 + t] != seg.none & 0xFFFF:
-                                assert x > j
-                                acc[x] = acc[x] - product.factor(op[x][2 + t]) * xj
-                else:
-                    assert all(w == seg.none for x in op for w in x[2 + used:])
-                    for x in range(32):
-                        for w in op[x][2:]:
-                            acc[x] = product(acc[x], w)
+                assert all(w == seg.none for x in op for w in x[2 + used:])
+                for x in range(32):
+                    for w in op[x][2:]:
+                        acc[x] = acc[x] - G[w & 0xFFFF] * X[w >> 16]
                 if ctl[0] & coop.L_END:
                     acc = _fold(acc, ctl)
                     done += [(x[0], x[1], acc[k]) for k, x in enumerate(op) if x[1] & coop.L_LEAD]
+                    assert bool(ctl[0] & coop.L_DIAGS) == any(x[1] & coop.L_DIAG for x in op)
                 sync = ctl[0] >> coop.L_SYNC
             wait[v] = max(sync - 1, 0)
             place[v] = (i, acc)
+        assert len({h & 0xFFFF for h, _, _ in done}) == len(done)
         for h, c, a in done:
-            finish(h & 0xFFFF, h >> 16, c, scale(h >> 16, c, a))
+            finish(h & 0xFFFF, h >> 16, c, a)
     assert not any(wait)
-
-
-class _Term:
-    def __init__(self, G, X):
-        self.G, self.X = G, X
-
-    def factor(self, p):
-        return self.G[p]
-
-    def __call__(self, acc, w):
-        return acc - self.G[w & 0xFFFF] * self.X[w >> 16]
 
 
 def _run(m, V, F, K, split, nw, ghinv, rhs):
@@ -178,44 +162,103 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
     _sums(segs["dest"], "dest",
           lambda a, w: a + (rx[w[0] & 0xFFFF] * xv[w[0] >> 16]) * xv[w[1]], set_x)
 
+    buf = Array([None] * p["buffer"], None)
+    if p["buffer"]:
+        for k, x in enumerate(_rates(segs["bufd"], prod4, p["nbufd"])):
+            buf[8 * k] = x
+
+    def singles(seg, area, put):
+        for op in (op for ops in segs[seg].ops for op in ops):
+            for x in op:
+                for k in range(0, 8, 2):
+                    if x[k] & 0xFFFF != coop.NO_ENTRY:
+                        put(x[k] & 0xFFFF, coef[x[k] >> 16] * area[x[k + 1]])
+
+    def put_buf(d, x):
+        assert buf[d] is None
+        buf[d] = x
+
+    def chain(first, blocks):
+        s = 0.0
+        for k in range(first, first + blocks * coop.BLOCK):
+            s = s + buf[8 * k]
+        return s
+
+    for i, first, blocks in p["chains"][0]:
+        set_x(8 * i, chain(first, blocks))
+
     def fin_prod(h, acc):
         X[h] = acc - X[h] * xv[h]
 
     _sums(segs["prod"], "sum", add(A), fin_prod)
+    if p["buffer"]:
+        singles("bufp", A, put_buf)
+        assert None not in buf.v[:-1]
+    for i, first, blocks in p["chains"][1]:
+        fin_prod(8 * i, chain(first, blocks))
     fun = np.array(X.v[:n])
-    G, R = Array([None] * nnz, 0.0), Array([None] * n, 1.0)
+    ng = p["ng"]
+    recip = ng - 1 - n
+    G = Array([None] * ng, 0.0, 1)
+    G[ng - 1] = -1.0
 
     def set_g(h, acc):
-        assert G[h] is None
-        G[h] = acc
+        assert G[h // 8] is None
+        G[h // 8] = acc
 
     for q in range(p["parts"]):
         B = Array(_rates(segs[f"bpart{q}"], prod4, p["nbp"][q]) + [None] * (nreact - p["nbp"][q]), 0.0)
         _sums(segs[f"jvs{q}"], "sum", add(B), set_g)
+        singles(f"one{q}", B, set_g)
     for i, (o, final) in enumerate(p["diag"]):
         G[o] = G[o] + ghinv
-        if final:
-            R[8 * i] = 1.0 / G[o] if G[o] else float("inf")
-    G0 = np.array(G.v[:nnz])
+        if final and split:
+            G[recip + i] = -1.0 / G[o] if G[o] else float("-inf")
+    tail, t0 = p["tail"], n - p["tail"]
+    block = [[p["block"] + i * tail + c for c in range(tail)] for i in range(tail)]
+    G0 = np.array([G[k] for k in p["factor"]])
 
-    def scale(r, c, acc):
-        if split:
-            return acc if c & coop.L_DIAG else acc * R[r]
-        return acc / G[p["diag"][r // 8][0]] if c & coop.L_SCALED else acc
-
-    def set_lu(d, r, c, acc):
-        G[d] = acc
+    def set_lu(d, e, c, acc):
         if c & coop.L_DIAG:
-            R[r] = 1.0 / acc if acc else float("inf")
+            if split:
+                G[e] = -1.0 / acc if acc else float("-inf")
+        elif split:
+            acc = -(acc * G[e])
+        elif c & coop.L_SCALED:
+            acc = acc / G[e]
+        G[d] = acc
 
-    _levels(segs["lu"], lambda d: G[d], _Term(G, G), scale, set_lu)
-    X = Array(rhs, 0.0)
+    _levels(segs["lu"], G, G, set_lu)
+    schur = np.array([[G[k] for k in row] for row in block]).reshape(tail, tail)
+    inv = schur.copy()
+    for k in range(tail):                     # Gauss-Jordan in place, no pivoting
+        row = inv[k] / inv[k, k]
+        row[k] = 1.0 / inv[k, k]
+        f = inv[:, k].copy()
+        inv[:, k] = 0.0
+        inv -= np.outer(f, row)
+        inv[k] = row
+    for i in range(tail):
+        for c in range(tail):
+            G[block[i][c]] = -inv[i, c]
+    X = Array(list(rhs) + [0.0] + [None] * (n + 1), None, 1)
 
-    def set_sweep(d, r, c, acc):
-        X[d] = acc
+    def set_sweep(d, e, c, acc):
+        assert d != n
+        X[d] = acc / G[e] if c & coop.L_SCALED else acc
 
-    _levels(segs["sweep"], lambda d: X[d], _Term(G, X), scale, set_sweep)
-    return fun, G0, np.array(G.v[:nnz]), np.array(X.v[:n])
+    _levels(segs["sweep"], G, X, set_sweep)
+    # the factors, the tail's from its Schur complement
+    lu = np.array([G[k] for k in p["factor"]])
+    for k in range(tail):
+        for i in range(k + 1, tail):
+            schur[i, k] /= schur[k, k]
+            schur[i, k + 1:] -= schur[i, k] * schur[k, k + 1:]
+    for q in range(nnz):
+        i, c = m["lu_irow"][q] - t0, m["lu_icol"][q] - t0
+        if tail and min(i, c) >= 0:
+            lu[q] = schur[i, c]
+    return fun, G0, lu, np.array([X[k] for k in p["place"]])
 
 
 def _oracle(name, m, V, F, K, ghinv, rhs):
@@ -244,10 +287,13 @@ def test_unsplit_streams_match_oracle_bits(case, nw):
 @pytest.mark.parametrize("nw", [4, 8])
 def test_split_streams_within_rounding(case, nw):
     """Componentwise rounding-error bounds (Higham, Accuracy and Stability of
-    Numerical Algorithms, ch. 3, 8 and 9), gamma_k = k u / (1 - k u):
-    a sum of k products is off by at most gamma_k of the sum of magnitudes,
-    the factorisation by gamma_n |L||U|, the solves by gamma_3n |L||U||x|.
-    Reciprocal pivots add one rounding to a multiplier and to a quotient."""
+    Numerical Algorithms, ch. 3, 8, 9 and 14), gamma_k = k u / (1 - k u):
+    a sum of k products is off by at most gamma_k of the sum of magnitudes and
+    the factorisation by gamma_n |L||U|.  A part's inverse formed by rows, and
+    the product with it, are off by gamma_n |M^-1||M||M^-1| for its block M, so
+    the solution by gamma |U^-1||L^-1||L||U||x| with the inverses of the
+    magnitudes' comparison matrices for |U^-1| and |L^-1|.  Reciprocal pivots
+    add a rounding to a multiplier and a quotient."""
     name, m, V, F, K = case
     n, crow, icol, irow = (m[k] for k in ("nvar", "lu_crow", "lu_icol", "lu_irow"))
     rhs = np.random.default_rng(5).standard_normal(n) * 1e5
@@ -278,9 +324,17 @@ def test_split_streams_within_rounding(case, nw):
         for p in range(crow[i], crow[i + 1]):
             (L if icol[p] < i else U)[i, icol[p]] = G[p]
     bound = np.abs(L) @ np.abs(U)
-    # the products L U and L U x are themselves formed in doubles here
+    # the product L U is itself formed in doubles here
     assert (np.abs(L @ U - A) <= gamma(2 * n + 8) * bound).all()
-    assert (np.abs(L @ (U @ x) - rhs) <= gamma(5 * n + 8) * (bound @ np.abs(x))).all()
+    ref = solve_triangular(U, solve_triangular(L, rhs, lower=True, unit_diagonal=True))
+    cL, cU = 2 * np.eye(n) - np.abs(L), 2 * np.diag(np.abs(np.diag(U))) - np.abs(U)
+
+    def inverse_magnitudes(v):
+        return solve_triangular(cU, solve_triangular(cL, v, lower=True))
+
+    reach = inverse_magnitudes(bound @ np.abs(ref) + np.abs(rhs))
+    assert (reach >= 0).all()
+    assert (np.abs(x - ref) <= gamma(8 * n) * reach).all()
 
 
 @pytest.mark.parametrize("split", [False, True])
