@@ -305,7 +305,7 @@ extern "C" cudaError_t rodas3_adjoint_launch(int ncell, const double* C0, const 
                                              const double* lam, double* gC0, double* gK,
                                              int* ierr, double* ws, long slots,
                                              int* sortbuf, unsigned long long* sortscratch,
-                                             cudaStream_t s) {
+                                             int coop_sms, cudaStream_t s) {
   AdjArgs a;
   a.ncell = ncell; a.C0 = C0; a.RCONST = RCONST; a.ISTAT = ISTAT; a.ckpt = ckpt;
   a.ckpt_max = ckpt_max; a.lam = lam; a.gC0 = gC0; a.gK = gK; a.ierr = ierr; a.ws = ws;
@@ -317,6 +317,9 @@ extern "C" cudaError_t rodas3_adjoint_launch(int ncell, const double* C0, const 
     if (e != cudaSuccess) return e;
     a.order = sortbuf + ncell;
   }
+  if (coop_sms > 0)      /* one block per cell on that many SMs */
+    return rodas3_coop_adjoint_launch(ncell, C0, RCONST, ISTAT, ckpt, ckpt_max, lam, gC0, gK, ierr,
+                                      a.order, coop_sms, s);
   const int threads = 128;
   for (long first = 0; first < ncell; first += slots) {
     const int count = (int)((ncell - first) < slots ? (ncell - first) : slots);

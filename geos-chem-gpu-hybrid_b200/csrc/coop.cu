@@ -494,6 +494,89 @@ __device__ __forceinline__ void coop_tail(double* sm) {
 }
 #endif
 
+/* Fun_SPLIT of the state in V into X; `after`: the segment that follows */
+template <int NT, int NG>
+__device__ __forceinline__ void coop_fun(unsigned int cell, CoopFetch& f, double* sm, int after) {
+  using L = CoopAt<NT>;
+  const int tid = threadIdx.x % NT;
+  (void)sm; (void)tid;
+  /* Fun_SPLIT: X = P_VAR - D_VAR*V; the destruction sums need no rates,
+     so they run before the barrier that publishes A */
+  coop_run<P_RATE, NT, NG>(cell, f, COOP_SEG_RATE, COOP_SEG_DEST, NREACT);
+#if COOP_BUFFER
+  coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_BUFD);
+  coop_run<P_BUFD, NT, NG>(cell, f, COOP_SEG_BUFD, COOP_SEG_PROD, COOP_NBUFD);
+  coop_sync<NT, NG>();
+  /* the last warp adds up the long destruction sums, then the first the
+     long production sums, which wait for all products */
+  const int lane = tid & 31;
+  if (tid >= NT - 32) {
+    const int i = __ldg(coop_chain_of + 3 * lane);
+    const double d = coop_chain<NT>(sm, __ldg(coop_chain_of + 3 * lane + 1), __ldg(coop_chain_of + 3 * lane + 2));
+    if (i >= 0) sm[L::X + i] = d;
+  }
+  coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, COOP_SEG_BUFP);
+  coop_run<P_BUFP, NT, NG>(cell, f, COOP_SEG_BUFP, after);
+  coop_sync<NT, NG>();
+  if (tid < 32) {
+    const int i = __ldg(coop_chain_of + 96 + 3 * lane);
+    const double p = coop_chain<NT>(sm, __ldg(coop_chain_of + 97 + 3 * lane), __ldg(coop_chain_of + 98 + 3 * lane));
+    if (i >= 0) sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i];
+  }
+#else
+  coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_PROD);
+  coop_sync<NT, NG>();
+  coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, after);
+#endif
+  coop_sync<NT, NG>();
+}
+
+/* -Jac0 + ghinv on the diagonal, into G; *ising (INT_MAX before) */
+template <int NT, int NG>
+__device__ __forceinline__ void coop_jacobian(unsigned int cell, CoopFetch& f, double* sm,
+                                              double ghinv, int* s_ising) {
+  using L = CoopAt<NT>;
+  constexpr int NE = (NVAR + NT - 1) / NT;
+  const int tid = threadIdx.x % NT;
+  /* Jac_SP straight into ros_PrepareMatrix's form: G = -JVS, a part of
+     the columns at a time, then ghinv on the diagonal.  KppDecomp's
+     singularity test reads each prepared diagonal before its row is
+     eliminated, so it is taken here: *ising becomes the lowest failing
+     row + 1.  Diagonals without updates are final: their reciprocals. */
+#pragma unroll 1
+  for (int q = 0; q < COOP_PARTS; ++q) {
+    const int seg = COOP_SEG_BPART0 + 3 * q;
+    coop_run<P_RATE, NT, NG>(cell, f, seg, seg + 1, COOP_NBP(q));
+    coop_sync<NT, NG>();
+    coop_run<P_JVS, NT, NG>(cell, f, seg + 1, seg + 2);
+    coop_run<P_ONE, NT, NG>(cell, f, seg + 2, q + 1 < COOP_PARTS ? seg + 3 : COOP_SEG_LU);
+    coop_sync<NT, NG>();
+  }
+#pragma unroll
+  for (int m = 0; m < NE; ++m) {
+    const int k = tid + m * NT;
+    if (k < NVAR) {
+      const int o = __ldg(coop_diag + k);
+      const double g = sm[L::G + (o >> 1)] + ghinv;
+      if (fabs(g) < DBL_MIN) atomicMin(s_ising, k + 1);
+      sm[L::G + (o >> 1)] = g;
+#if COOP_SPLIT
+      if (o & 1) sm[L::G + L::RECIP + k] = -1.0 / g;
+#endif
+    }
+  }
+  coop_sync<NT, NG>();
+}
+
+template <int NT, int NG>
+__device__ __forceinline__ void coop_factor(unsigned int cell, CoopFetch& f, double* sm) {
+  /* KppDecomp entry by entry, in levels */
+  coop_run<P_LU, NT, NG>(cell, f, COOP_SEG_LU, COOP_SEG_SWEEP);
+#if COOP_TAIL
+  coop_tail<NT, NG>(sm);
+#endif
+}
+
 /* load the cell's column and set the integrator state (lane_start of the
    one-thread-per-cell kernels); attempt 1 is the retry: Hstart taken as 0
    and the retry tolerances */
@@ -645,68 +728,12 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
       }
       if (s >= 2) c.st.nfun += 1;
       coop_sync<NT, NG>();
-      /* Fun_SPLIT: X = P_VAR - D_VAR*V; the destruction sums need no rates,
-         so they run before the barrier that publishes A */
-      const int after = s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP;
-      coop_run<P_RATE, NT, NG>(cell, f, COOP_SEG_RATE, COOP_SEG_DEST, NREACT);
-#if COOP_BUFFER
-      coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_BUFD);
-      coop_run<P_BUFD, NT, NG>(cell, f, COOP_SEG_BUFD, COOP_SEG_PROD, COOP_NBUFD);
-      coop_sync<NT, NG>();
-      /* the last warp adds up the long destruction sums, then the first the
-         long production sums, which wait for all products */
-      const int lane = tid & 31;
-      if (tid >= NT - 32) {
-        const int i = __ldg(coop_chain_of + 3 * lane);
-        const double d = coop_chain<NT>(sm, __ldg(coop_chain_of + 3 * lane + 1), __ldg(coop_chain_of + 3 * lane + 2));
-        if (i >= 0) sm[L::X + i] = d;
-      }
-      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, COOP_SEG_BUFP);
-      coop_run<P_BUFP, NT, NG>(cell, f, COOP_SEG_BUFP, after);
-      coop_sync<NT, NG>();
-      if (tid < 32) {
-        const int i = __ldg(coop_chain_of + 96 + 3 * lane);
-        const double p = coop_chain<NT>(sm, __ldg(coop_chain_of + 97 + 3 * lane), __ldg(coop_chain_of + 98 + 3 * lane));
-        if (i >= 0) sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i];
-      }
-#else
-      coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_PROD);
-      coop_sync<NT, NG>();
-      coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, after);
-#endif
-      coop_sync<NT, NG>();
+      coop_fun<NT, NG>(cell, f, sm, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
     }
     if (s == -1) {
 #pragma unroll
       for (int m = 0; m < NE; ++m) f0[m] = tid + m * NT < NVAR ? sm[L::X + tid + m * NT] : 0.0;
-      /* Jac_SP straight into ros_PrepareMatrix's form: G = -JVS, a part of
-         the columns at a time, then ghinv on the diagonal.  KppDecomp's
-         singularity test reads each prepared diagonal before its row is
-         eliminated, so it is taken here: *ising becomes the lowest failing
-         row + 1.  Diagonals without updates are final: their reciprocals. */
-#pragma unroll 1
-      for (int q = 0; q < COOP_PARTS; ++q) {
-        const int seg = COOP_SEG_BPART0 + 3 * q;
-        coop_run<P_RATE, NT, NG>(cell, f, seg, seg + 1, COOP_NBP(q));
-        coop_sync<NT, NG>();
-        coop_run<P_JVS, NT, NG>(cell, f, seg + 1, seg + 2);
-        coop_run<P_ONE, NT, NG>(cell, f, seg + 2, q + 1 < COOP_PARTS ? seg + 3 : COOP_SEG_LU);
-        coop_sync<NT, NG>();
-      }
-#pragma unroll
-      for (int m = 0; m < NE; ++m) {
-        const int k = tid + m * NT;
-        if (k < NVAR) {
-          const int o = __ldg(coop_diag + k);
-          const double g = sm[L::G + (o >> 1)] + ghinv;
-          if (fabs(g) < DBL_MIN) atomicMin(s_ising, k + 1);
-          sm[L::G + (o >> 1)] = g;
-#if COOP_SPLIT
-          if (o & 1) sm[L::G + L::RECIP + k] = -1.0 / g;
-#endif
-        }
-      }
-      coop_sync<NT, NG>();
+      coop_jacobian<NT, NG>(cell, f, sm, ghinv, s_ising);
       c.st.ndec += 1;
       if (*s_ising != INT_MAX) {
         c.st.nsng += 1;
@@ -717,11 +744,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
         c.ierr = -8;
         return 1;
       }
-      /* KppDecomp entry by entry, in levels */
-      coop_run<P_LU, NT, NG>(cell, f, COOP_SEG_LU, COOP_SEG_SWEEP);
-#if COOP_TAIL
-      coop_tail<NT, NG>(sm);
-#endif
+      coop_factor<NT, NG>(cell, f, sm);
       continue;
     }
 #pragma unroll
@@ -899,6 +922,17 @@ __global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 2) rodas3_coop(CoopArgs 
   }
 }
 
+#if COOP_SPLIT
+#include "coop_adjoint.cuh"
+#else
+extern "C" int rodas3_coop_adjoint_ok(void) { return 0; }
+extern "C" cudaError_t rodas3_coop_adjoint_launch(int, const double*, const double*, const int*,
+                                                  const double*, int, const double*, double*,
+                                                  double*, int*, const int*, int, cudaStream_t) {
+  return cudaErrorInvalidValue;
+}
+#endif
+
 static size_t coop_smem_bytes(int threads, int cells) {
   const int cell = threads == 128 ? CoopAt<128>::CELL : CoopAt<256>::CELL;
   return ((size_t)cells * cell + COOP_NCOEF) * sizeof(double);
@@ -972,7 +1006,13 @@ extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bp
 extern "C" int rodas3_coop_ok(void) { return 0; }
 extern "C" size_t rodas3_coop_smem_bytes(void) { return 0; }
 extern "C" int rodas3_coop_blocks_per_sm(int) { return 0; }
-extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch*, int, cudaStream_t) {
+extern "C" int rodas3_coop_adjoint_ok(void) { return 0; }
+extern "C" cudaError_t rodas3_coop_adjoint_launch(int, const double*, const double*, const int*,
+                                                  const double*, int, const double*, double*,
+                                                  double*, int*, const int*, int, cudaStream_t) {
+  return cudaErrorInvalidValue;
+}
+extern "C" cudaError_t rodas3_coop_launch(const Rodas3Launch*, int, int, cudaStream_t) {
   return cudaErrorInvalidValue;
 }
 

@@ -477,18 +477,25 @@ int gcchem_b200_adjoint_device(int nCell, const double* C0, const double* RCONST
   DevState& s = g_dev[d];
   std::lock_guard<std::mutex> lock(s.mu);
   if (ensure_init(s, d) != 0) return -1;
-  const long per = (long)rodas3_adjoint_ws_elems() * 8;
-  long slots = round_up(nCell, 32);
-  size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
-    long cap = (long)((double)fr * 0.5 / (double)per) / 32 * 32;
-    if (cap < 32) cap = 32;
-    if (slots > cap) slots = cap;
-  }
-  if (slots > s.aws_slots) {
-    if (s.aws) { cudaFree(s.aws); s.aws = nullptr; s.aws_slots = 0; }
-    if (cudaMalloc(&s.aws, (size_t)slots * per) != cudaSuccess) { cudaGetLastError(); return -2; }
-    s.aws_slots = slots;
+  /* one block per cell up to the same line as the forward solve: 24 cells
+     0.010 / 0.98 s, 6,000 cells 0.45 / 1.9 s, 15,900 cells (60 s step) 0.93 / 2.0 s against
+     one thread per cell; a plain launch mode keeps the latter */
+  const bool coop = s.mode != RODAS3_PLAIN && s.mode != RODAS3_PLAIN_FUSED &&
+                    rodas3_coop_adjoint_ok() && (nCell <= kCoopCells || !rodas3_fused_lu());
+  if (!coop) {
+    const long per = (long)rodas3_adjoint_ws_elems() * 8;
+    long slots = round_up(nCell, 32);
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
+      long cap = (long)((double)fr * 0.5 / (double)per) / 32 * 32;
+      if (cap < 32) cap = 32;
+      if (slots > cap) slots = cap;
+    }
+    if (slots > s.aws_slots) {
+      if (s.aws) { cudaFree(s.aws); s.aws = nullptr; s.aws_slots = 0; }
+      if (cudaMalloc(&s.aws, (size_t)slots * per) != cudaSuccess) { cudaGetLastError(); return -2; }
+      s.aws_slots = slots;
+    }
   }
   if (nCell > s.asort_n) {
     if (s.asort) { cudaFree(s.asort); s.asort = nullptr; s.asort_n = 0; }
@@ -500,7 +507,7 @@ int gcchem_b200_adjoint_device(int nCell, const double* C0, const double* RCONST
   }
   if (ensure_sortc(s, nCell) != 0) return -2;
   return rodas3_adjoint_launch(nCell, C0, RCONST, ISTAT, ckpt, ckpt_max, lam, gC0, gK, ierr,
-                               s.aws, s.aws_slots, s.asort, s.sortc,
+                               s.aws, s.aws_slots, s.asort, s.sortc, coop ? s.sm_count : 0,
                                (cudaStream_t)stream) == cudaSuccess ? 0 : -3;
 }
 

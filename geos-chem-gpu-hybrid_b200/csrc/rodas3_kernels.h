@@ -49,6 +49,12 @@ int rodas3_coop_ok(void);
 size_t rodas3_coop_smem_bytes(void);
 int rodas3_coop_blocks_per_sm(int threads);
 cudaError_t rodas3_coop_launch(const Rodas3Launch* L, int sms, int bps, cudaStream_t s);
+/* its adjoint (production build): order as in rodas3_adjoint_launch */
+int rodas3_coop_adjoint_ok(void);
+cudaError_t rodas3_coop_adjoint_launch(int ncell, const double* C0, const double* RCONST,
+                                       const int* ISTAT, const double* ckpt, int ckpt_max,
+                                       const double* lam, double* gC0, double* gK, int* ierr,
+                                       const int* order, int sms, cudaStream_t s);
 double rodas3_fp64_peak_tflops(void);
 long rodas3_cost_scratch(int n);
 cudaError_t rodas3_cost_order(const int* keys, int n, int* order,
@@ -59,7 +65,7 @@ cudaError_t rodas3_adjoint_launch(int ncell, const double* C0, const double* RCO
                                   const int* ISTAT, const double* ckpt, int ckpt_max,
                                   const double* lam, double* gC0, double* gK, int* ierr,
                                   double* ws, long slots, int* sortbuf,
-                                  unsigned long long* sortscratch, cudaStream_t s);
+                                  unsigned long long* sortscratch, int coop_sms, cudaStream_t s);
 cudaError_t rodas3_perm_to_order(const int* perm, int n, int* order, int* bad,
                                  cudaStream_t s);
 

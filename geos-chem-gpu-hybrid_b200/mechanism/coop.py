@@ -296,6 +296,12 @@ OP_COST, TERM_COST, FOLD_COST, END_COST = 250, 25, 45, 60
 
 BLOCK = 8              # terms that a chain adds between two tests of its length
 NO_ENTRY = 0xFFFF      # single operations: an idle pair
+# The discrete adjoint adds four segments: the transposed sweeps (U^T, then L^T;
+# the parts in reverse, each [terms outside the part, product with the
+# transposed inverse]), t_j = S_j . u per reaction (tj), the partials
+# dA(j)/dV(i) of every rate (apart), and per species the sums of t_j times a
+# partial and of t_j times its derivative along a stage vector (vthl).
+
 LONG = 30              # terms of Fun's sums above which a sum goes through the buffer
 
 
@@ -682,10 +688,31 @@ def level_programs(mech: dict, split: bool, nw: int):
     for q in range(len(bpart)):
         segs[f"one{q}"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(segs[f"one{q}"])
     segs["lu"], segs["sweep"] = best["lu"], best["sweep"]
+    extra_of = [j for j, _ in extra]
+    scoef, apart, by_species = {1.0: 0}, [], [[] for _ in range(n)]
+    if split:
+        one_x = n + nfix
+        for j, f in enumerate(rate):
+            for k in (1, 2, 3):
+                if f[k] < n:
+                    rest = [x for q, x in enumerate(f) if q not in (0, k)]
+                    by_species[f[k]].append(8 * j | 8 * len(apart) << 16)
+                    apart.append([f[0]] + rest + [one_x])
+        react = [[] for _ in range(nreact)]
+        for i, j, v in mech["stoich"]:
+            react[j].append(8 * slot(scoef, float(codegen.literal(v))) | 8 * i << 16)
+        if 8 * len(apart) >= 1 << 16:
+            return None
+        segs["sweept"] = best["sweept"]
+        segs["tj"] = Segment(nw, 8 * n << 16).sums([((8 * j, 0), w) for j, w in enumerate(react)], True)
+        segs["apart"] = Segment(nw, no_rate, None).rates([words4(f) for f in apart])
+        segs["vthl"] = Segment(nw, 8 * nreact | 8 * len(apart) << 16).sums(
+            [((8 * i, 0), w) for i, w in enumerate(by_species)], True)
     return {"segs": segs, "parts": len(parts), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
             "nbp": [len(part) for part in parts], "ng": best["ng"], "place": best["place"], "tail": tail,
             "chains": chains, "buffer": len(rates_d) + len(ones_p), "nbufd": len(rates_d), "factor": place, "block": block, "diag": [(at_diag[i], i < t0 and not upd[diag[i]]) for i in range(n)],
-            "cost": best["cost"]}
+            "cost": best["cost"], "scoef": scoef, "napart": len(apart), "place_t": best["place_t"],
+            "has_k": [int(f[0] < nreact or extra_of[f[0] - nreact] >= 0) for f in rate]}
 
 
 # most entries that a part's inverse may add; every pair is tried
@@ -809,7 +836,59 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
                          for i in range(t0, n)], split)
             x = x[:t0] + new[t0:]
     lu.pad(), sweep.pad()
-    return {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
+    out = {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
+    if limits is not None and not estimate:
+        out["sweept"], out["place_t"] = _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw)
+    else:
+        out["place_t"] = x
+    return out
+
+
+def _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw):
+    """The sweeps with the transposed matrix on the same factors and inverses."""
+    t0, minus, zero = n - tail, rbase + n, rbase + n + 1
+    seg = Segment(nw, zero | n << 16, n | minus << 16)
+    x = list(range(n))
+
+    def columns(deps):
+        cols = [[] for _ in range(n)]
+        for i in range(n):
+            for c, p in deps[i]:
+                cols[c].append((i, p))
+        return cols
+
+    def outside(rows, cols, done):
+        out = [((x[c] | minus << 16, L_START), [p | x[i] << 16 for i, p in cols[c] if done(i)]) for c in rows]
+        out = [it for it in out if it[1]]
+        if out:
+            seg.level(out, split)
+
+    def product(items):
+        """items {row: words}: the rows' values go to their other place."""
+        nonlocal x
+        new = list(x)
+        for j in items:
+            new[j] = (x[j] + n + 1) % (2 * n + 2)
+        if items:
+            seg.level([((new[j] | minus << 16, 0), w) for j, w in items.items()], split)
+        x = new
+
+    for parts, deps, scaled in ((bwd, upper, True), (fwd, lower, False)):
+        cols = columns(deps)
+        for rows, reach in reversed(parts):
+            inside = set(rows)
+            outside(rows, cols, lambda i: i not in inside)
+            of = {j: [] for j in rows}
+            for i in rows:
+                for j in reach[i]:
+                    of[j].append(at[(i, j)] | x[i] << 16)
+            product({j: [(rbase + j if scaled else minus) | x[j] << 16] + of[j]
+                     for j in rows if scaled or of[j]})
+        if tail and scaled:
+            outside(range(t0, n), cols, lambda i: i < t0)
+            product({j: [block + (i - t0) * tail + j - t0 | x[i] << 16 for i in range(t0, n)]
+                     for j in range(t0, n)})
+    return seg.pad(), x
 
 
 EARLY = 2              # levels between an early product's readiness and its sum's end
@@ -845,6 +924,8 @@ def coop_inc(mech: dict) -> str:
                           doubles("coop_extra_val", [v for _, v in p["extra"]]),
                           f"#define COOP_NCOEF {len(p['coef']) + len(p['coef']) % 2}",
                           doubles("coop_coef", list(p["coef"]) + [0.0] * (len(p["coef"]) % 2)),
+                          f"#define COOP_NAPART {p['napart']}", f"#define COOP_NSCOEF {len(p['scoef'])}",
+                          doubles("coop_scoef", p["scoef"]), arr("unsigned char", "coop_has_k", p["has_k"]),
                           f"#define COOP_BUFFER {p['buffer']}", f"#define COOP_NBUFD {p['nbufd']}",
                           arr("int", "coop_chain_of", [x for c in p["chains"] for k in range(32)
                                                     for x in (c[k] if k < len(c) else (-1, 0, 0))]),
@@ -852,7 +933,7 @@ def coop_inc(mech: dict) -> str:
                               [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),
                           arr("int", "coop_diag", [o << 1 | (e and 1) for o, e in p["diag"]])]
                 lines += [f"#define COOP_SEG_{name.upper()} {k}" for k, name in enumerate(p["segs"])]
-            lines += [f"#define COOP_NG{nw} {p['ng']}", arr("int", f"coop_place{nw}", p["place"])]
+            lines += [arr("int", f"coop_place_t{nw}", p["place_t"]), f"#define COOP_NG{nw} {p['ng']}", arr("int", f"coop_place{nw}", p["place"])]
             words, where = [], []
             for seg in p["segs"].values():
                 for ops in seg.ops:
