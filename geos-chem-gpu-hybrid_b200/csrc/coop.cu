@@ -1,51 +1,47 @@
 /*
  * coop.cu -- the cooperative Rodas3 kernel: one thread block per cell, the
- * whole cell state in shared memory.
+ * whole cell state on chip.
  *
- * The one-thread-per-cell kernels stream every cell's workspace (the LU
- * factors, the Jacobian, the stage vectors) through HBM, because 256 cells
- * per SM cannot keep 50-125 KB each on chip.  Here a block of 128 or 256
- * threads owns one cell at a time and keeps its factors G (NNZ doubles), the
- * state and stage vectors, the rate constants and a scratch array in shared
- * memory (69 KB for the 120-species synthetic mechanism, 94 KB for
- * fullchem), so the solve reads HBM only to load a cell and store its
- * result.  The block drains the same cost-ordered work queue as the
- * persistent kernel: thread 0 takes the next queue position, and the block
- * solves that cell to the end (with the in-place retry), then takes the next.
+ * One thread per cell is right when hundreds of thousands of cells hide the
+ * latency of each other's workspace accesses.  A small batch cannot: a thread
+ * needs 2.5-4 ms for one attempt of a step (B200, fullchem, any batch of up to
+ * a few thousand cells), whatever the GPU has idle.  Here a group of 128 or 256
+ * threads owns one cell: the factors, the vectors, the rate constants and the
+ * rates are in shared memory (106 KB for fullchem), the state and the stage
+ * vectors in registers, so a solve reads HBM only to load a cell and store its
+ * result, and an attempt takes 72 us.  A block holds one cell, or two when
+ * there are more cells than SMs.  The groups drain the same cost-ordered queue
+ * as the persistent kernel.
  *
- * Parallelism inside a cell comes from tables generated from the mechanism
- * (coop.inc, mechanism/coop.py):
- *   Fun      rates A(j) one per thread, then P_VAR/D_VAR/Vdot one species per
- *            thread (gckpp_Function.F90:2170-5060 expressions, same rounding);
- *   Jac      partials B(m), then entries JVS(k), written straight into the
- *            factor array as -JVS (+ 1/(H*gamma) on the diagonal); the
- *            Jacobian is recomputed at every attempt instead of being stored
- *            (Y is unchanged after a rejection, so it is the same Jacobian);
- *   KppDecomp right-looking: step j forms column j's multipliers, then
- *            applies pivot row j to every row below it at once; each entry
- *            gets its updates in the reference's order
- *            (gckpp_LinearAlgebra.F90:46-84), so the factors are identical;
- *   KppSolve forward sweep by columns, each row's terms in the reference's
- *            order (:645-2311); backward sweep by levels of rows in the
- *            reference's order (--fmad=false build), or by columns (FMA
- *            build: 120 parallel steps instead of a chain of every row's
- *            terms, the per-row order reversed).
+ * Parallelism inside a cell comes from the instruction streams that
+ * mechanism/coop.py generates (coop.inc), one list of operations per warp:
+ *   Fun      rates A(j), then the destruction and production sums, each in the
+ *            reference's order in one lane (gckpp_Function.F90:2170-5060); the
+ *            few long ones from a buffer of their products;
+ *   Jac      partials B(m), then the entries, straight into the factor array
+ *            as -JVS, + 1/(H*gamma) on the diagonal; formed again at every
+ *            attempt instead of stored (Y is unchanged after a rejection);
+ *   KppDecomp by dependency levels: an entry's updates, in the reference's
+ *            order (gckpp_LinearAlgebra.F90:46-84), as soon as their factors
+ *            are final;
+ *   KppSolve by levels of rows (:645-2311).
+ * The FMA build (COOP_SPLIT) may round differently: there sums other than
+ * Fun's are split over lanes, quotients become products with one reciprocal
+ * per pivot (GC_IRECIP), the last rows are inverted as a block (coop_tail) and
+ * the sweeps use inverses of their diagonal blocks, 22 levels in place of 130.
+ * Built with --fmad=false the kernel reproduces the CPU oracle bit for bit.
+ *
  * Step-size control, counters, options and the retry protocol are the
  * arithmetic of Integrate_Cell_S (gckpp_BatchIntegrator.F90:408-707) and of
  * the model's retry (fullchem_mod.F90:2436-2520), computed redundantly by
- * every thread of the block so that every branch is block-uniform; the one
- * sequential sum (the error norm, in species order) is taken by thread 0.
+ * every thread of the cell so that every branch is uniform.
  *
- * Built with --fmad=false this kernel reproduces the CPU oracle bit for bit,
- * as the one-thread-per-cell kernels do; the FMA build contracts into FMA
- * and forms the multipliers and the backward quotients from one reciprocal
- * per pivot (GC_IRECIP).
- *
- * Every __syncthreads() is reached by all threads of the block: loop bounds
- * come from the tables, and every branch around a barrier depends only on
+ * Every barrier of a cell is reached by all threads of its group: the streams
+ * of all warps hold the same number of barriers between two phases (checked by
+ * the generator's test), and every branch around a barrier depends only on
  * values all threads hold identically (shared-memory words read after a
  * barrier, or scalars computed redundantly from them).  Nothing waits on
- * another block.
+ * another block, nor on the block's other cell.
  */
 #include <cuda_runtime.h>
 #include <float.h>
@@ -134,7 +130,11 @@ struct CoopCell {
    and the programs have few levels.  One cell, fullchem, time of an attempt on
    a B200: rounds of the whole block with words loaded one round ahead 185 us;
    streams 118 us; with inverses of the sweeps' parts and of the tail block
-   (13 + 9 levels instead of 61 + 69) 86 us. */
+   (13 + 9 levels instead of 61 + 69) 86 us; with byte offsets, six products to
+   an operation of Fun and a buffer without bank conflicts 72 us (137,000 cycles:
+   ~85,000 warp instructions in four warps, 6-7 cycles each; the FP64 pipe is
+   used at 3%).  Two cells in a block share the schedulers' gaps: 290 cells take
+   78 us per attempt, 16,000 cells 3.4 M attempts per second. */
 struct CoopFetch {
   uint4 q[COOP_DEPTH][2];
 };
@@ -241,28 +241,32 @@ __device__ __forceinline__ void coop_rate_op(unsigned int cell, uint4 a, uint4 b
                       ((f[k][0] * f[k][1]) * f[k][2]) * f[k][3]);
 }
 
-/* three products of a destruction sum */
-template <int NT>
-__device__ __forceinline__ double coop_dest_op(unsigned int cell, double acc, uint4 a, uint4 b) {
-  const unsigned int w[6] = {a.z, a.w, b.x, b.y, b.z, b.w}, u = coop_uniform(a.y & CL_UNIFORM);
-  double f[3], h[3], g[3];
+/* six products of a sum that one lane adds up in order (dest, prod) */
+template <int PROG, int NT>
+__device__ __forceinline__ double coop_line_op(unsigned int cell, unsigned int coef, double acc,
+                                               uint4 qa, uint4 qb) {
+  using L = CoopAt<NT>;
+  const unsigned int w[6] = {qa.z, qa.w, qb.x, qb.y, qb.z, qb.w}, u = coop_uniform(qa.y & CL_UNIFORM);
+  double a[6], b[6];
 #pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    f[t] = coop_get<CoopAt<NT>::RX>(cell, w[2 * t] & 0xFFFFu);
-    h[t] = coop_get<CoopAt<NT>::V>(cell, w[2 * t] >> 16);
-    g[t] = coop_get<CoopAt<NT>::V>(cell, w[2 * t + 1]);
+  for (int t = 0; t < 6; ++t) {
+    a[t] = PROG == P_DEST ? coop_get<L::RX>(cell, w[t] & 0xFFFFu) : coop_get<0>(coef, w[t] & 0xFFFFu);
+    b[t] = coop_get<PROG == P_DEST ? L::V : L::A>(cell, w[t] >> 16);
   }
   if (u & CL_FIRST) acc = 0.0;
 #pragma unroll
-  for (int t = 0; t < 3; ++t) acc = acc + (f[t] * h[t]) * g[t];
+  for (int t = 0; t < 6; ++t) acc = acc + a[t] * b[t];
   if (u & CL_END) {
-    coop_put_if<CoopAt<NT>::X>(a.y & CL_LEAD, cell, a.x, acc);
+    const unsigned int d = qa.x & 0xFFFFu;
+    double x = acc;
+    if (PROG == P_PROD) x = acc - coop_get<L::X>(cell, d) * coop_get<L::V>(cell, d);
+    coop_put_if<L::X>(qa.y & CL_LEAD, cell, d, x);
   }
   return acc;
 }
 
 /* half of a sum operation: three products, then perhaps the entry's end */
-template <int PROG, int NT>
+template <int NT>
 __device__ __forceinline__ double coop_sum_half(unsigned int cell, unsigned int coef, double acc,
                                                 uint4 q) {
   const unsigned int w[3] = {q.y, q.z, q.w}, ctl = q.x >> 16, d = q.x & 0xFFFFu;
@@ -277,13 +281,8 @@ __device__ __forceinline__ double coop_sum_half(unsigned int cell, unsigned int 
 #pragma unroll
   for (int t = 0; t < 3; ++t) acc = acc + a[t] * b[t];
   if (u & CL_END) {
-    if (PROG == P_JVS) acc = coop_fold(acc, ctl, (u >> 9) & 7u);
-    if (PROG == P_PROD) {
-      const double x = coop_get<CoopAt<NT>::X>(cell, d), v = coop_get<CoopAt<NT>::V>(cell, d);
-      coop_put_if<CoopAt<NT>::X>(ctl & CL_LEAD, cell, d, acc - x * v);
-    } else {
-      coop_put_if<CoopAt<NT>::G>(ctl & CL_LEAD, cell, d, acc);
-    }
+    acc = coop_fold(acc, ctl, (u >> 9) & 7u);
+    coop_put_if<CoopAt<NT>::G>(ctl & CL_LEAD, cell, d, acc);
   }
   return acc;
 }
@@ -305,20 +304,19 @@ __device__ __forceinline__ void coop_one_op(unsigned int cell, unsigned int coef
   }
 }
 
-/* level operation of the factorisation (P_LU) or a sweep; operands are element
-   indices */
+/* level operation of the factorisation (P_LU) or a sweep */
 template <int PROG, int NT, int NG>
 __device__ __forceinline__ double coop_level_op(unsigned int cell, double acc, uint4 qa, uint4 qb) {
   using L = CoopAt<NT>;
   constexpr int BASE = PROG == P_LU ? L::G : L::X;
-  const unsigned int ctl = qa.y, d = 8u * (qa.x & 0xFFFFu), e = 8u * (qa.x >> 16);
+  const unsigned int ctl = qa.y, d = qa.x & 0xFFFFu, e = qa.x >> 16;
   const unsigned int u = coop_uniform(ctl & CL_UNIFORM);
   const unsigned int w[6] = {qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
   double a[6], b[6];
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
-    a[t] = coop_get<L::G>(cell, 8u * (w[t] & 0xFFFFu));
-    b[t] = coop_get<BASE>(cell, 8u * (w[t] >> 16));
+    a[t] = coop_get<L::G>(cell, w[t] & 0xFFFFu);
+    b[t] = coop_get<BASE>(cell, w[t] >> 16);
   }
   if (u & CL_FIRST) {
     acc = 0.0;
@@ -328,8 +326,8 @@ __device__ __forceinline__ double coop_level_op(unsigned int cell, double acc, u
   if (u & (4u << 12)) {                    /* more than three products */
 #pragma unroll
     for (int t = 3; t < 6; ++t) {
-      a[t] = coop_get<L::G>(cell, 8u * (w[t] & 0xFFFFu));
-      b[t] = coop_get<BASE>(cell, 8u * (w[t] >> 16));
+      a[t] = coop_get<L::G>(cell, w[t] & 0xFFFFu);
+      b[t] = coop_get<BASE>(cell, w[t] >> 16);
     }
 #pragma unroll
     for (int t = 0; t < 6; ++t) acc = acc - a[t] * b[t];
@@ -390,13 +388,13 @@ __device__ __forceinline__ void coop_run(unsigned int cell, CoopFetch& f, int se
         j += 4 * NT;
       } else if (PROG == P_ONE || PROG == P_BUFP) {
         coop_one_op<NT, PROG == P_ONE ? CoopAt<NT>::G : CoopAt<NT>::B>(cell, coef, a, b);
-      } else if (PROG == P_DEST) {
-        acc = coop_dest_op<NT>(cell, acc, a, b);
+      } else if (PROG == P_DEST || PROG == P_PROD) {
+        acc = coop_line_op<PROG, NT>(cell, coef, acc, a, b);
       } else if (PROG == P_LU || PROG == P_SWEEP) {
         acc = coop_level_op<PROG, NT, NG>(cell, acc, a, b);
       } else {
-        acc = coop_sum_half<PROG, NT>(cell, coef, acc, a);
-        acc = coop_sum_half<PROG, NT>(cell, coef, acc, b);
+        acc = coop_sum_half<NT>(cell, coef, acc, a);
+        acc = coop_sum_half<NT>(cell, coef, acc, b);
       }
       /* into the registers just read: a load into others would be copied at
          the end of the loop, and the copy would wait for it */
@@ -494,12 +492,21 @@ __device__ __forceinline__ void coop_tail(double* sm) {
 }
 #endif
 
+/* a thread's long sum: the first warp's are productions, the last's destructions */
+template <int NT>
+__device__ __forceinline__ void coop_chain_load(int* chain) {
+  const int tid = threadIdx.x % NT, k = 3 * (tid & 31) + (tid < 32 ? 96 : 0);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) chain[t] = coop_chain_of[k + t];
+}
+
 /* Fun_SPLIT of the state in V into X; `after`: the segment that follows */
 template <int NT, int NG>
-__device__ __forceinline__ void coop_fun(unsigned int cell, CoopFetch& f, double* sm, int after) {
+__device__ __forceinline__ void coop_fun(unsigned int cell, CoopFetch& f, double* sm,
+                                         const int* chain, int after) {
   using L = CoopAt<NT>;
   const int tid = threadIdx.x % NT;
-  (void)sm; (void)tid;
+  (void)sm; (void)tid; (void)chain;
   /* Fun_SPLIT: X = P_VAR - D_VAR*V; the destruction sums need no rates,
      so they run before the barrier that publishes A */
   coop_run<P_RATE, NT, NG>(cell, f, COOP_SEG_RATE, COOP_SEG_DEST, NREACT);
@@ -509,18 +516,16 @@ __device__ __forceinline__ void coop_fun(unsigned int cell, CoopFetch& f, double
   coop_sync<NT, NG>();
   /* the last warp adds up the long destruction sums, then the first the
      long production sums, which wait for all products */
-  const int lane = tid & 31;
   if (tid >= NT - 32) {
-    const int i = __ldg(coop_chain_of + 3 * lane);
-    const double d = coop_chain<NT>(sm, __ldg(coop_chain_of + 3 * lane + 1), __ldg(coop_chain_of + 3 * lane + 2));
-    if (i >= 0) sm[L::X + i] = d;
+    const double d = coop_chain<NT>(sm, chain[1], chain[2]);
+    if (chain[0] >= 0) sm[L::X + chain[0]] = d;
   }
   coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, COOP_SEG_BUFP);
   coop_run<P_BUFP, NT, NG>(cell, f, COOP_SEG_BUFP, after);
   coop_sync<NT, NG>();
   if (tid < 32) {
-    const int i = __ldg(coop_chain_of + 96 + 3 * lane);
-    const double p = coop_chain<NT>(sm, __ldg(coop_chain_of + 97 + 3 * lane), __ldg(coop_chain_of + 98 + 3 * lane));
+    const int i = chain[0];
+    const double p = coop_chain<NT>(sm, chain[1], chain[2]);
     if (i >= 0) sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i];
   }
 #else
@@ -678,7 +683,8 @@ __device__ __forceinline__ double coop_root(double x) {
    step_prologue, step_factor and step_stages in rodas3_kernels.cu. */
 template <int NT, int NG>
 __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, CoopFetch& f,
-                                            unsigned int cell, double* sm, double* y, const int* place) {
+                                            unsigned int cell, double* sm, double* y, const int* place,
+                                            const int* chain) {
   using L = CoopAt<NT>;
   const int tid = threadIdx.x % NT;
   constexpr int NE = (NVAR + NT - 1) / NT;      /* species of a thread */
@@ -728,7 +734,7 @@ __device__ __forceinline__ int coop_attempt(CoopCell& c, const CoopArgs& a, Coop
       }
       if (s >= 2) c.st.nfun += 1;
       coop_sync<NT, NG>();
-      coop_fun<NT, NG>(cell, f, sm, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
+      coop_fun<NT, NG>(cell, f, sm, chain, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
     }
     if (s == -1) {
 #pragma unroll
@@ -878,7 +884,8 @@ __global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 2) rodas3_coop(CoopArgs 
   __shared__ unsigned int s_pos[NG];
   const int g = NG == 1 ? 0 : threadIdx.x / NT, tid = threadIdx.x % NT;
   double* sm = reinterpret_cast<double*>(coop_smem) + COOP_NCOEF + g * CoopAt<NT>::CELL;
-  const unsigned int cell = (unsigned int)__cvta_generic_to_shared(sm);
+  /* warp-uniform, so that it is added by the load itself */
+  const unsigned int cell = __reduce_max_sync(0xFFFFFFFFu, (unsigned int)__cvta_generic_to_shared(sm));
   for (int i = threadIdx.x; i < COOP_NCOEF; i += NT * NG)
     reinterpret_cast<double*>(coop_smem)[i] = coop_coef[i];
   if (tid == 0) {
@@ -896,6 +903,8 @@ __global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 2) rodas3_coop(CoopArgs 
 #pragma unroll
   for (int m = 0; m < NE; ++m)
     place[m] = tid + m * NT < NVAR ? (NT == 128 ? coop_place4 : coop_place8)[tid + m * NT] : NVAR;
+  int chain[3];
+  coop_chain_load<NT>(chain);
   int have = 0, drained = 0;
   for (;;) {
     while (!have && !drained) {
@@ -915,7 +924,7 @@ __global__ void __launch_bounds__(NT * NG, NG > 1 ? 1 : 2) rodas3_coop(CoopArgs 
     } else if (!have) {
       break;
     }
-    if (have && coop_attempt<NT, NG>(c, a, f, cell, sm, y, place)) {
+    if (have && coop_attempt<NT, NG>(c, a, f, cell, sm, y, place, chain)) {
       have = !coop_end<NT, NG>(c, a, sm, y);
       coop_sync<NT, NG>();    /* the result is stored before the next cell loads */
     }

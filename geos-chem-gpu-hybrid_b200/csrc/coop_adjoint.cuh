@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128, 1) rodas3_coop_adjoint(CoopAdjArgs a) {
   constexpr int NT = 128, NE = (NVAR + NT - 1) / NT;
   const int tid = threadIdx.x;
   double* sm = reinterpret_cast<double*>(coop_smem) + COOP_NCOEF;
-  const unsigned int cell = (unsigned int)__cvta_generic_to_shared(sm);
+  const unsigned int cell = __reduce_max_sync(0xFFFFFFFFu, (unsigned int)__cvta_generic_to_shared(sm));
   int* s_ising = reinterpret_cast<int*>(sm + L::RED + 8);
   for (int i = tid; i < COOP_NCOEF; i += NT) reinterpret_cast<double*>(coop_smem)[i] = coop_coef[i];
   for (int i = tid; i < COOP_NSCOEF; i += NT) sm[L::SC + i] = coop_scoef[i];
@@ -176,6 +176,8 @@ __global__ void __launch_bounds__(128, 1) rodas3_coop_adjoint(CoopAdjArgs a) {
     place[m] = tid + m * NT < NVAR ? coop_place4[tid + m * NT] : NVAR;
     place_t[m] = tid + m * NT < NVAR ? coop_place_t4[tid + m * NT] : NVAR;
   }
+  int chain[3];
+  coop_chain_load<NT>(chain);
   CoopFetch f;
   coop_prime<NT, 1>(f, COOP_SEG_RATE);
   for (int q = blockIdx.x; q < a.ncell; q += gridDim.x) {
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(128, 1) rodas3_coop_adjoint(CoopAdjArgs a) {
             if (tid + m * NT < NVAR) sm[L::V + tid + m * NT] = ys[m];
           }
           __syncthreads();
-          coop_fun<NT, 1>(cell, f, sm, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
+          coop_fun<NT, 1>(cell, f, sm, chain, s == -1 ? COOP_SEG_BPART0 : COOP_SEG_SWEEP);
         }
         if (s == -1) {
 #pragma unroll

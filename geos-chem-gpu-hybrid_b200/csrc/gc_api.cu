@@ -8,8 +8,8 @@
  *   2. returns at once when nCell <= 0,
  *   3. checks Perm on the host (IERR(:) = -100 for an entry outside 1..nCell)
  *      and copies C, RCONST, ATOL, RTOL, ICNTRL, RCNTRL and Perm to the device,
- *   4. runs the solve (persistent queue kernel by default; GCCHEM_B200_MODE=
- *      plain selects the one-thread-per-cell kernel),
+ *   4. runs the solve (the kernel that auto_mode picks; GCCHEM_B200_MODE or
+ *      set_launch name another),
  *   5. copies C, ISTAT, RSTAT and IERR back,
  * and reports tTotal (whole call) and tKernel (solve kernels, CUDA events).
  * Unlike the reference, device buffers and the solver workspace are cached
@@ -42,14 +42,14 @@ const int kAuto = -1;
 /* The cooperative kernel solves a cell in a thirtieth of the time one thread
    takes, but keeps only two cells per SM; one thread per cell catches up once
    the batch fills the GPU several times.  Full cold steps on a B200,
-   cooperative / persistent: fullchem 1 cell 0.009 / 0.262 s, 1,000 cells 0.030 /
-   0.549 s, 16,000 cells 0.47 / 1.05 s, 29,952 cells 0.88 / 1.25 s, 238,464
-   cells 2.9 M / 4.6 M attempts per second.  The line is drawn below the
+   cooperative / persistent: fullchem 1 cell 0.008 / 0.27 s, 1,000 cells 0.026 /
+   0.549 s, 16,000 cells 0.41 / 1.08 s, 29,952 cells 0.76 / 1.25 s, 238,464
+   cells 3.4 M / 4.6 M attempts per second.  The line is drawn below the
    crossover (about 50,000 cells): one cell in 10^5 has a step-size sequence that
    amplifies any difference in rounding to 1e-8 and more, so that only batches
    that gain at least twofold leave the arithmetic of the thread-per-cell
    kernels.  Without the fused factorisation (synthetic mechanism) the
-   cooperative kernel wins at every size: 1,500 cells 0.022 / 0.66 s, 2.3 M /
+   cooperative kernel wins at every size: 1,500 cells 0.020 / 0.66 s, 2.4 M /
    0.8 M attempts per second at full load.  The --fmad=false build may not
    split sums over lanes: 100 cells 0.14 / 0.56 s, even at about 1,000. */
 #if defined(GC_LU_RECIP) && GC_LU_RECIP

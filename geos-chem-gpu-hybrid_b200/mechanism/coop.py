@@ -231,23 +231,21 @@ def compile_tables(mech: dict):
 # the warp executes them.  The addresses of a stream are known in advance, so
 # the kernel fetches operations several ahead of their use.
 #
-# Rates and sums give operands as byte offsets in their array (the kernel keeps
-# the cell in shared memory), level operations as element indices; a missing
-# operand is the index of a constant 0 (or 1) behind the array, so that it
-# needs no test.
+# Operands are given as byte offsets in their array (the kernel keeps the cell
+# in shared memory), so that a word needs no arithmetic; a missing operand
+# points at a constant 0 (or 1) behind the array, so that it needs no test.
 #
 #   rate operations   four products (f0 | f1<<16, f2 | f3<<16).  Product k of
 #                     operation i of warp w and lane l is number
 #                     ((i*4 + k)*NW + w)*32 + l.
-#   dest operations   header, control, three products (f0 | f1<<16, f2)
-#   sum operations    two halves of a header and three words (prod, jvs)
+#   sum operations    two halves of a header and three words (jvs)
 #   single operations four pairs (entry | coefficient<<16, partial)
-#   level operations  header, control, six words (lu, sweep)
+#   level operations  header, control, six words (dest, prod, lu, sweep)
 #
 # Control word, per lane: L_* flags, log2 of the lane's group, exchanges that
 # the warp does (the largest of its groups), products in use, block barriers
 # after the operation.  A sum's header is its entry's offset | control << 16; a
-# level's is the entry's index | the index of its scale << 16.
+# level's is the entry's offset | the offset of its scale << 16.
 #
 # The sweeps of the production build use partitioned inverses (Alvarado and
 # Schreiber, Optimal parallel solution of sparse triangular systems, 1993):
@@ -302,7 +300,7 @@ NO_ENTRY = 0xFFFF      # single operations: an idle pair
 # dA(j)/dV(i) of every rate (apart), and per species the sums of t_j times a
 # partial and of t_j times its derivative along a stage vector (vthl).
 
-LONG = 30              # terms of Fun's sums above which a sum goes through the buffer
+LONG = 60              # terms of Fun's sums above which a sum goes through the buffer
 
 
 def _lanes(items, k, split):
@@ -394,12 +392,13 @@ class Segment:
                     out.append((self.head, ctl, [self.none] * per_op))
             yield out
 
-    def dest(self, items, split):
-        warps, self.cost = _place(items, self.nw, split, 3)
+    def lines(self, items):
+        """Sums of one lane each, six products an operation; no barrier."""
+        warps, self.cost = _place(items, self.nw, False, 6)
         for v, rounds in enumerate(warps):
             for lanes in rounds:
-                for op in self._split(lanes, 3):
-                    self.ops[v].append([[h, c] + [x for w in ws for x in w] for h, c, ws in op])
+                for op in self._split(lanes, 6):
+                    self.ops[v].append([[h, c] + w for h, c, w in op])
         return self.pad()
 
     def sums(self, items, split):
@@ -433,6 +432,16 @@ class Segment:
                 for op in self._split(lanes, 6):
                     self.ops[v].append([[h, c | diags] + w for h, c, w in op])
         self._sync()
+
+    def in_bytes(self):
+        """Element indices (both halves of headers and words) as offsets."""
+        for ops in self.ops:
+            for op in ops:
+                for lane in op:
+                    lane[0] *= 8
+                    lane[2:] = [8 * w for w in lane[2:]]
+        self.none *= 8
+        return self.pad()
 
     def _sync(self):
         """A block barrier after everything so far."""
@@ -602,18 +611,15 @@ def level_programs(mech: dict, split: bool, nw: int):
     def words4(f):
         return [8 * f[0] | 8 * f[1] << 16, 8 * f[2] | 8 * f[3] << 16]
 
-    def dword(f):          # (f0*f1)*f2, with the constant 1 in the middle of k*v
-        p, q = (f[2], f[1]) if f[2] == n + nfix else (f[1], f[2])
-        return (8 * f[0] | 8 * p << 16, 8 * q)
-
     def scaled_words(words):
         return [8 * (w & 0xFFFF) | 8 * (w >> 16) << 16 for w in words]
 
-    no_rate, no_dest, no_sum = (zero | one << 16, one | one << 16), (zero | one << 16, one), 8 * nreact << 16
+    no_rate, no_sum = (zero | one << 16, one | one << 16), 8 * nreact << 16
     segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
             "dest": None, "bufd": None, "prod": None, "bufp": None}
-    long_d = [i for i, w in dest if split and len(w) > LONG]
-    long_p = [i for i, w in prod if split and (len(w) > LONG or i in long_d)]
+    # a destruction term of three factors has no place in a line's words
+    long_d = [i for i, w in dest if len(w) > LONG and split or any(f[2] != n + nfix and f[1] != n + nfix for f in w)]
+    long_p = [i for i, w in prod if len(w) > LONG and split or i in long_d]
     if len(long_p) > 32:
         return None
     # the buffer: the long sums' products, each sum padded to whole blocks
@@ -621,7 +627,9 @@ def level_programs(mech: dict, split: bool, nw: int):
 
     def buffer(key, sums, none, at):
         out = []
-        for i, words in sums:
+        for c, (i, words) in enumerate(sums):
+            # the lanes' pairs of products start in different banks
+            out += [none] * ((2 * c - at - len(out)) % 16)
             first[(key, i)] = (at + len(out), -(-len(words) // BLOCK))
             out += words + [none] * (-len(words) % BLOCK)
         return out
@@ -630,12 +638,11 @@ def level_programs(mech: dict, split: bool, nw: int):
     ones_p = buffer("p", [(i, scaled_words(w)) for i, w in prod if i in long_p], no_sum, len(rates_d))
     if not long_p:
         del segs["bufd"], segs["bufp"]
-    segs["dest"] = Segment(nw, no_dest).dest([((8 * i, 0), [dword(f) for f in w])
-                                              for i, w in dest if i not in long_d], False)
+    segs["dest"] = Segment(nw, zero | one << 16).lines([((8 * i, 0), [8 * f[0] | 8 * (f[1] if f[2] == n + nfix else f[2]) << 16
+                                                                     for f in w]) for i, w in dest if i not in long_d])
     if long_p:
         segs["bufd"] = Segment(nw, no_rate, None).rates(rates_d)
-    segs["prod"] = Segment(nw, no_sum).sums([((8 * i, 0), scaled_words(w))
-                                             for i, w in prod if i not in long_p], False)
+    segs["prod"] = Segment(nw, no_sum).lines([((8 * i, 0), scaled_words(w)) for i, w in prod if i not in long_p])
     if long_p:
         segs["bufp"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(
             [(8 * (len(rates_d) + k), w) for k, w in enumerate(ones_p)])
@@ -682,6 +689,11 @@ def level_programs(mech: dict, split: bool, nw: int):
     limits = None
     if split:
         tried = [(f, u) for f in INVERSE_LIMITS for u in INVERSE_LIMITS]
+        # (the offsets of the factor array have to fit 16 bits)
+        tried = [lim for lim in tried if 8 * _factor_and_sweeps(
+            n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["ng"] < 1 << 16]
+        if not tried:
+            return None
         limits = min(tried, key=lambda lim: _factor_and_sweeps(
             n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["cost"])
     best = _factor_and_sweeps(n, tail, block, entries, at_diag, lower, upper, split, nw, limits)
@@ -835,7 +847,7 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
                           [block + (i - t0) * tail + j - t0 | x[j] << 16 for j in range(t0, n)])
                          for i in range(t0, n)], split)
             x = x[:t0] + new[t0:]
-    lu.pad(), sweep.pad()
+    lu.pad().in_bytes(), sweep.pad().in_bytes()
     out = {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
     if limits is not None and not estimate:
         out["sweept"], out["place_t"] = _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw)
@@ -888,7 +900,7 @@ def _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw):
             outside(range(t0, n), cols, lambda i: i < t0)
             product({j: [block + (i - t0) * tail + j - t0 | x[i] << 16 for i in range(t0, n)]
                      for j in range(t0, n)})
-    return seg.pad(), x
+    return seg.pad().in_bytes(), x
 
 
 EARLY = 2              # levels between an early product's readiness and its sum's end

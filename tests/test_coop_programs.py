@@ -29,19 +29,19 @@ def case(request):
 
 
 class Array:
-    """Elements addressed by byte offset (unit 8) or index (unit 1); the one
-    behind the last may not be written."""
+    """Elements addressed by byte offset; the one behind the last may not be
+    written."""
 
-    def __init__(self, values, last, unit=8):
-        self.v, self.unit = list(values) + [last], unit
+    def __init__(self, values, last):
+        self.v = list(values) + [last]
 
     def __getitem__(self, off):
-        assert off % self.unit == 0
-        return self.v[off // self.unit]
+        assert off % 8 == 0
+        return self.v[off // 8]
 
     def __setitem__(self, off, x):
-        assert off % self.unit == 0 and off // self.unit < len(self.v) - 1
-        self.v[off // self.unit] = x
+        assert off % 8 == 0 and off // 8 < len(self.v) - 1
+        self.v[off // 8] = x
 
 
 def _rates(seg, product, n):
@@ -73,8 +73,8 @@ def _sum_steps(seg, kind):
     for ops in seg.ops:
         yield None
         for op in ops:
-            if kind == "dest":
-                yield [(x[0], x[1], [(x[2 + 2 * t], x[3 + 2 * t]) for t in range(3)]) for x in op]
+            if kind == "line":
+                yield [(x[0], x[1], x[2:]) for x in op]
             else:
                 for h in (0, 4):
                     yield [(x[h] & 0xFFFF, x[h] >> 16, x[h + 1:h + 4]) for x in op]
@@ -159,8 +159,7 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
         assert X[h] is None
         X[h] = acc
 
-    _sums(segs["dest"], "dest",
-          lambda a, w: a + (rx[w[0] & 0xFFFF] * xv[w[0] >> 16]) * xv[w[1]], set_x)
+    _sums(segs["dest"], "line", lambda a, w: a + rx[w & 0xFFFF] * xv[w >> 16], set_x)
 
     buf = Array([None] * p["buffer"], None)
     if p["buffer"]:
@@ -190,7 +189,7 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
     def fin_prod(h, acc):
         X[h] = acc - X[h] * xv[h]
 
-    _sums(segs["prod"], "sum", add(A), fin_prod)
+    _sums(segs["prod"], "line", add(A), fin_prod)
     if p["buffer"]:
         singles("bufp", A, put_buf)
         assert None not in buf.v[:-1]
@@ -199,24 +198,24 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
     fun = np.array(X.v[:n])
     ng = p["ng"]
     recip = ng - 1 - n
-    G = Array([None] * ng, 0.0, 1)
-    G[ng - 1] = -1.0
+    G = Array([None] * ng, 0.0)
+    G[8 * ng - 8] = -1.0
 
     def set_g(h, acc):
-        assert G[h // 8] is None
-        G[h // 8] = acc
+        assert G[h] is None
+        G[h] = acc
 
     for q in range(p["parts"]):
         B = Array(_rates(segs[f"bpart{q}"], prod4, p["nbp"][q]) + [None] * (nreact - p["nbp"][q]), 0.0)
         _sums(segs[f"jvs{q}"], "sum", add(B), set_g)
         singles(f"one{q}", B, set_g)
     for i, (o, final) in enumerate(p["diag"]):
-        G[o] = G[o] + ghinv
+        G[8 * o] = G[8 * o] + ghinv
         if final and split:
-            G[recip + i] = -1.0 / G[o] if G[o] else float("-inf")
+            G[8 * (recip + i)] = -1.0 / G[8 * o] if G[8 * o] else float("-inf")
     tail, t0 = p["tail"], n - p["tail"]
-    block = [[p["block"] + i * tail + c for c in range(tail)] for i in range(tail)]
-    G0 = np.array([G[k] for k in p["factor"]])
+    block = [[8 * (p["block"] + i * tail + c) for c in range(tail)] for i in range(tail)]
+    G0 = np.array([G[8 * k] for k in p["factor"]])
 
     def set_lu(d, e, c, acc):
         if c & coop.L_DIAG:
@@ -241,15 +240,15 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
     for i in range(tail):
         for c in range(tail):
             G[block[i][c]] = -inv[i, c]
-    X = Array(list(rhs) + [0.0] + [None] * (n + 1), None, 1)
+    X = Array(list(rhs) + [0.0] + [None] * (n + 1), None)
 
     def set_sweep(d, e, c, acc):
-        assert d != n
+        assert d != 8 * n
         X[d] = acc / G[e] if c & coop.L_SCALED else acc
 
     _levels(segs["sweep"], G, X, set_sweep)
     # the factors, the tail's from its Schur complement
-    lu = np.array([G[k] for k in p["factor"]])
+    lu = np.array([G[8 * k] for k in p["factor"]])
     for k in range(tail):
         for i in range(k + 1, tail):
             schur[i, k] /= schur[k, k]
@@ -258,7 +257,7 @@ def _run(m, V, F, K, split, nw, ghinv, rhs):
         i, c = m["lu_irow"][q] - t0, m["lu_icol"][q] - t0
         if tail and min(i, c) >= 0:
             lu[q] = schur[i, c]
-    return fun, G0, lu, np.array([X[k] for k in p["place"]])
+    return fun, G0, lu, np.array([X[8 * k] for k in p["place"]])
 
 
 def _oracle(name, m, V, F, K, ghinv, rhs):
