@@ -42,21 +42,23 @@ const int kAuto = -1;
 /* The cooperative kernel solves a cell in a thirtieth of the time one thread
    takes, but keeps only two cells per SM; one thread per cell catches up once
    the batch fills the GPU several times.  Full cold steps on a B200,
-   cooperative / persistent: fullchem 1 cell 0.008 / 0.27 s, 1,000 cells 0.026 /
-   0.549 s, 16,000 cells 0.41 / 1.08 s, 29,952 cells 0.76 / 1.25 s, 238,464
-   cells 3.4 M / 4.6 M attempts per second.  The line is drawn below the
-   crossover (about 50,000 cells): one cell in 10^5 has a step-size sequence that
+   cooperative / persistent: fullchem 1 cell 0.008 / 0.27 s, 1,000 cells 0.033 /
+   0.555 s, 16,000 cells 0.41 / 1.08 s, 29,952 cells 0.76 / 1.19 s; at full load
+   3.4 M / 4.6 M attempts per second.  The line is drawn below the crossover
+   (about 50,000 cells): one cell in 10^5 has a step-size sequence that
    amplifies any difference in rounding to 1e-8 and more, so that only batches
    that gain at least twofold leave the arithmetic of the thread-per-cell
    kernels.  Without the fused factorisation (synthetic mechanism) the
    cooperative kernel wins at every size: 1,500 cells 0.020 / 0.66 s, 2.4 M /
    0.8 M attempts per second at full load.  The --fmad=false build may not
-   split sums over lanes: 100 cells 0.14 / 0.56 s, even at about 1,000. */
+   split sums over lanes, and its two kernels give the same bits: fullchem 100
+   cells 0.11 / 0.58 s, 1,000 cells 0.24 / 0.76 s, 4,000 cells 0.76 / 1.18 s, 8,000
+   cells 1.46 / 1.30 s; synthetic 1,500 cells 0.24 / 0.74 s. */
 #if defined(GC_LU_RECIP) && GC_LU_RECIP
 const int kCoopCells = 16000;
 const bool kCoopAlways = true;      /* without the fused factorisation */
 #else
-const int kCoopCells = 1000;
+const int kCoopCells = 4000;
 const bool kCoopAlways = false;
 #endif
 
