@@ -49,7 +49,7 @@ const int kAuto = -1;
    amplifies any difference in rounding to 1e-8 and more, so that only batches
    that gain at least twofold leave the arithmetic of the thread-per-cell
    kernels.  Without the fused factorisation (synthetic mechanism) the
-   cooperative kernel wins at every size: 1,500 cells 0.020 / 0.66 s, 2.4 M /
+   cooperative kernel wins at every size: 1,500 cells 0.019 / 0.66 s, 2.6 M /
    0.8 M attempts per second at full load.  The --fmad=false build may not
    split sums over lanes, and its two kernels give the same bits: fullchem 100
    cells 0.11 / 0.58 s, 1,000 cells 0.24 / 0.76 s, 4,000 cells 0.76 / 1.18 s, 8,000

@@ -303,9 +303,13 @@ NO_ENTRY = 0xFFFF      # single operations: an idle pair
 LONG = 60              # terms of Fun's sums above which a sum goes through the buffer
 
 
-def _lanes(items, k, split):
+def _lanes(items, k, split, dense=False):
     """Warp rounds of one level: [(header, words)] -> lists of at most 32
-    (header, log2 group, words of the lane), groups aligned to their size."""
+    (header, log2 group, words of the lane), groups aligned to their size.
+    dense: the items are rows of the tail block, a multiple of 16 doubles apart;
+    each starts with another column, or all rows' entries of a column, which are
+    in one bank of shared memory, would be read together (synthetic mechanism:
+    13,400 passes of a half warp's loads per attempt in the sweeps, 6,200 so)."""
     sized = []
     for head, words in items:
         g = 1
@@ -318,6 +322,9 @@ def _lanes(items, k, split):
         if len(lanes) + g > 32:
             rounds.append(lanes)
             lanes = []
+        if dense:
+            turn = len(lanes) % len(words)
+            words = words[turn:] + words[:turn]
         lanes += [(head, g.bit_length() - 1, words[q::g]) for q in range(g)]
     if lanes:
         rounds.append(lanes)
@@ -330,13 +337,13 @@ def _cost(lanes, per_op):
     return OP_COST * max(1, -(-k // per_op)) + TERM_COST * k + FOLD_COST * s + END_COST
 
 
-def _place(items, nw, split, per_op):
+def _place(items, nw, split, per_op, dense=False):
     """A level's rounds on nw warps: (warp lists, cost of the longest)."""
     best, cost = None, None
     longest = max([len(w) for _, w in items] + [1])
     for k in (range(1, min(longest, 40) + 1) if split else (longest,)):
         warps, load = [[] for _ in range(nw)], [0] * nw
-        for lanes in sorted(_lanes(items, k, split), key=lambda r: -_cost(r, per_op)):
+        for lanes in sorted(_lanes(items, k, split, dense), key=lambda r: -_cost(r, per_op)):
             w = load.index(min(load))
             warps[w].append(lanes)
             load[w] += _cost(lanes, per_op)
@@ -423,8 +430,8 @@ class Segment:
             self.ops[v][w // 4][n % 32][w % 4 * 2:w % 4 * 2 + 2] = [head | (word & 0xFFFF) << 16, word >> 16]
         return self.pad()
 
-    def level(self, items, split):
-        warps, cost = _place(items, self.nw, split, 6)
+    def level(self, items, split, dense=False):
+        warps, cost = _place(items, self.nw, split, 6, dense)
         self.cost += cost + 30
         for v, rounds in enumerate(warps):
             for lanes in rounds:
@@ -845,7 +852,7 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
             new = [i if i < t0 else i + n + 1 for i in range(n)]
             sweep.level([((new[i] | minus << 16, 0),
                           [block + (i - t0) * tail + j - t0 | x[j] << 16 for j in range(t0, n)])
-                         for i in range(t0, n)], split)
+                         for i in range(t0, n)], split, True)
             x = x[:t0] + new[t0:]
     lu.pad().in_bytes(), sweep.pad().in_bytes()
     out = {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
