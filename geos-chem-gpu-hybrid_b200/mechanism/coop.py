@@ -1,10 +1,14 @@
-"""Tables for the cooperative kernel (one thread block per cell).
+"""Programs for the cooperative kernel (one thread block per cell).
 
 The one-thread-per-cell kernels run straight-line statement lists.  In the
-cooperative kernel the threads of a block share one cell, so every thread
-runs the same instructions on different entries: Fun, Jac, the
-factorisation and the solves become loops over tables.  This module turns
-the mechanism IR into those tables; ``coop_inc`` emits them as C arrays.
+cooperative kernel the warps of a block share one cell, and each executes its
+own list of operations on the cell's arrays.  ``level_programs`` turns the
+mechanism IR into those lists, ``coop_inc`` emits them as C arrays.  The two
+forms (split or not), the levels, the inverses of the sweeps and the format of
+the words are described where they are built.
+
+``compile_tables`` holds the expressions themselves as flat tables; it decides
+whether a mechanism's expressions have a shape that the programs support.
 
 Expressions.  Every rate A(j), production P_VAR(i), destruction D_VAR(i),
 Jacobian partial B(m) and entry JVS(k) of the IR is a left-associated
@@ -20,28 +24,11 @@ the --fmad=false build rounds like them.  A mechanism with any other
 expression shape gets no tables (``compile_tables`` returns None) and no
 cooperative kernel.
 
-Factorisation (KppDecomp, gckpp_LinearAlgebra.F90:46-84), right-looking.
-The reference eliminates row by row: row k receives, in increasing pivot
-order j, ``W(c) = W(c) + a*U(j,c)`` with ``a = -(W(j)/U(j,j))``, and stores
-``-a`` as L(k,j).  Step j of the right-looking form first forms the
-multipliers of column j (every row i > j with L(i,j) in the pattern) and
-then applies pivot row j to all those rows at once.  Each entry still
-receives its updates in increasing pivot order and the same operations, so
-the result is the same bit for bit; the parallelism is the rows and columns
-of one step instead of one row's columns.
-
-Solves (KppSolve, gckpp_LinearAlgebra.F90:645-2311).  The forward sweep
-``X(i) = X(i) - L(i,j)*X(j)`` over increasing j is run column by column:
-at step j, X(j) is final and every row i with L(i,j) subtracts its term --
-the same per-row order.  The backward sweep subtracts U(i,c)*X(c) in
-increasing c and then divides; its rows are grouped into levels (a row's
-level is one more than the highest level among its columns), rows of one
-level run in parallel, each row's terms in the reference order.  That
-order makes the sweep a chain of every row's terms (2,452 dependent
-subtractions for the synthetic mechanism), so the FMA build, which need
-not round like the reference, runs the backward sweep by columns too
-(``bwc``: at step i, X(i) = acc(i)/U(i,i) and every row r < i with U(r,i)
-subtracts its term), in the reverse of the reference's per-row order.
+Factorisation and solves.  Each entry of KppDecomp
+(gckpp_LinearAlgebra.F90:46-84) receives its updates in increasing pivot order,
+each row of KppSolve (:645-2311) its terms in the reference's order, with the
+same operations: the results of the unsplit programs are the reference's bit
+for bit, whatever the order in which independent entries are formed.
 """
 from __future__ import annotations
 
