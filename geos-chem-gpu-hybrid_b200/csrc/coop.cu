@@ -7,7 +7,7 @@
  * needs 2.5-4 ms for one attempt of a step (B200, fullchem, any batch of up to
  * a few thousand cells), whatever the GPU has idle.  Here a group of 128 or 256
  * threads owns one cell: the factors, the vectors, the rate constants and the
- * rates are in shared memory (106 KB for fullchem), the state and the stage
+ * rates are in shared memory (110 KB for fullchem), the state and the stage
  * vectors in registers, so a solve reads HBM only to load a cell and store its
  * result, and an attempt takes 72 us.  A block holds one cell, or two when
  * there are more cells than SMs.  The groups drain the same cost-ordered queue
