@@ -45,6 +45,14 @@ class Unsupported(ValueError):
     pass
 
 
+def _pack(lo, hi):
+    """Two 16-bit fields of a word; a field that does not fit must not spill
+    into the other."""
+    if not (0 <= lo < 1 << 16 and 0 <= hi < 1 << 16):
+        raise Unsupported("offset of more than 16 bits")
+    return lo | hi << 16
+
+
 def _factors(node, consts):
     """Factor codes of a left-associated product chain."""
     out = []
@@ -403,7 +411,7 @@ class Segment:
             if len(halves) % 2:
                 halves.append(idle)
             for a, b in zip(halves[::2], halves[1::2]):
-                self.ops[v].append([[h | (c & 0xFFF) << 16] + w + [g | (d & 0xFFF) << 16] + u
+                self.ops[v].append([[_pack(h, c & 0xFFF)] + w + [_pack(g, d & 0xFFF)] + u
                                     for (h, c, w), (g, d, u) in zip(a, b)])
         return self.pad([self.head] + [self.none] * 3 + [self.head] + [self.none] * 3)
 
@@ -414,7 +422,7 @@ class Segment:
             v, w = n // 32 % self.nw, n // (32 * self.nw)
             if w % 4 == 0 and len(self.ops[v]) == w // 4:
                 self.ops[v].append([self.idle() for _ in range(32)])
-            self.ops[v][w // 4][n % 32][w % 4 * 2:w % 4 * 2 + 2] = [head | (word & 0xFFFF) << 16, word >> 16]
+            self.ops[v][w // 4][n % 32][w % 4 * 2:w % 4 * 2 + 2] = [_pack(head, word & 0xFFFF), word >> 16]
         return self.pad()
 
     def level(self, items, split, dense=False):
@@ -429,12 +437,15 @@ class Segment:
 
     def in_bytes(self):
         """Element indices (both halves of headers and words) as offsets."""
+        def offsets(w):
+            return _pack(8 * (w & 0xFFFF), 8 * (w >> 16))
+
         for ops in self.ops:
             for op in ops:
                 for lane in op:
-                    lane[0] *= 8
-                    lane[2:] = [8 * w for w in lane[2:]]
-        self.none *= 8
+                    lane[0] = offsets(lane[0])
+                    lane[2:] = [offsets(w) for w in lane[2:]]
+        self.none = offsets(self.none)
         return self.pad()
 
     def _sync(self):
@@ -480,15 +491,22 @@ def _parts(n, deps, order, limit):
 
 
 def level_programs(mech: dict, split: bool, nw: int):
-    """The cooperative kernel's programs, or None for unsupported expression
-    shapes.  split: sums may be divided over lanes (production build); nw:
-    warps of the block."""
-    if compile_tables(mech) is None:
+    """The cooperative kernel's programs, or None for expression shapes or
+    sizes that they do not hold.  split: sums may be divided over lanes
+    (production build); nw: warps of the block."""
+    try:
+        return _programs(mech, split, nw)
+    except Unsupported:
         return None
+
+
+def _programs(mech, split, nw):
+    if compile_tables(mech) is None:
+        raise Unsupported("expression shape")
     n, nfix, nnz, nreact = mech["nvar"], mech["nfix"], mech["nnz"], mech["nreact"]
     crow, diag, icol, where = mech["lu_crow"], mech["lu_diag"], mech["lu_icol"], mech["lu_where"]
-    if 8 * nnz >= 1 << 16:             # byte offsets of 16 bits
-        return None
+    if 8 * nnz >= 1 << 16:
+        raise Unsupported("factors beyond 16-bit offsets")
     extra = {}                 # first factors behind the rate constants: (reaction or
                                # -1, literal), the literal itself or RCT(j)*literal
     ext = {1.0: 0}             # constants behind the species (other factors)
@@ -556,7 +574,7 @@ def level_programs(mech: dict, split: bool, nw: int):
                 c, t = c * float(codegen.literal(t[1][1])), t[2]
             if t[0] != tag:
                 raise Unsupported(str(t))
-            words.append(slot(coef, c) | index(t[1]) << 16)
+            words.append(_pack(slot(coef, c), index(t[1])))
         return words
 
     try:
@@ -594,28 +612,28 @@ def level_programs(mech: dict, split: bool, nw: int):
             dest.append((i, words))
         prod = [(i, scaled(e, "a", lambda j: j)) for i, e in enumerate(mech["prod"])]
         jvs = [scaled(e, "b", lambda j: bmap[j], -1.0) for e in mech["jvs"]]
-    except (Unsupported, KeyError):
-        return None
+    except KeyError as e:
+        raise Unsupported(f"missing partial {e}") from None
     nx = n + nfix + len(ext)
     zero = 8 * (nreact + len(extra))     # the constant 0 behind [RCT | extra]
     one = 8 * (n + nfix)
     if max(8 * nx, zero, 8 * len(coef)) >= 1 << 16:
-        return None
+        raise Unsupported("vectors beyond 16-bit offsets")
 
     def words4(f):
-        return [8 * f[0] | 8 * f[1] << 16, 8 * f[2] | 8 * f[3] << 16]
+        return [_pack(8 * f[0], 8 * f[1]), _pack(8 * f[2], 8 * f[3])]
 
     def scaled_words(words):
-        return [8 * (w & 0xFFFF) | 8 * (w >> 16) << 16 for w in words]
+        return [_pack(8 * (w & 0xFFFF), 8 * (w >> 16)) for w in words]
 
-    no_rate, no_sum = (zero | one << 16, one | one << 16), 8 * nreact << 16
+    no_rate, no_sum = (_pack(zero, one), _pack(one, one)), _pack(0, 8 * nreact)
     segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
             "dest": None, "bufd": None, "prod": None, "bufp": None}
     # a destruction term of three factors has no place in a line's words
     long_d = [i for i, w in dest if len(w) > LONG and split or any(f[2] != n + nfix and f[1] != n + nfix for f in w)]
     long_p = [i for i, w in prod if len(w) > LONG and split or i in long_d]
     if len(long_p) > 32:
-        return None
+        raise Unsupported("more than 32 long sums")
     # the buffer: the long sums' products, each sum padded to whole blocks
     first = {}
 
@@ -632,8 +650,9 @@ def level_programs(mech: dict, split: bool, nw: int):
     ones_p = buffer("p", [(i, scaled_words(w)) for i, w in prod if i in long_p], no_sum, len(rates_d))
     if not long_p:
         del segs["bufd"], segs["bufp"]
-    segs["dest"] = Segment(nw, zero | one << 16).lines([((8 * i, 0), [8 * f[0] | 8 * (f[1] if f[2] == n + nfix else f[2]) << 16
-                                                                     for f in w]) for i, w in dest if i not in long_d])
+    segs["dest"] = Segment(nw, _pack(zero, one)).lines(
+        [((8 * i, 0), [_pack(8 * f[0], 8 * (f[1] if f[2] == n + nfix else f[2])) for f in w])
+         for i, w in dest if i not in long_d])
     if long_p:
         segs["bufd"] = Segment(nw, no_rate, None).rates(rates_d)
     segs["prod"] = Segment(nw, no_sum).lines([((8 * i, 0), scaled_words(w)) for i, w in prod if i not in long_p])
@@ -664,7 +683,7 @@ def level_programs(mech: dict, split: bool, nw: int):
         if in_tail[p]:
             place[p] = block + (row_of[p] - t0) * tail + icol[p] - t0
     if 2 * tail > nreact or 8 * (block + tail * tail) > NO_ENTRY:
-        return None
+        raise Unsupported("tail block")
     # -Jac0 (the coefficients carry the sign); the kernel adds ghinv to the
     # diagonal and forms the reciprocals of the diagonals without updates
     fill = set(range(block, block + tail * tail)) - {place[p] for p in range(nnz)}
@@ -687,7 +706,7 @@ def level_programs(mech: dict, split: bool, nw: int):
         tried = [lim for lim in tried if 8 * _factor_and_sweeps(
             n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["ng"] < 1 << 16]
         if not tried:
-            return None
+            raise Unsupported("inverses beyond 16-bit offsets")
         limits = min(tried, key=lambda lim: _factor_and_sweeps(
             n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["cost"])
     best = _factor_and_sweeps(n, tail, block, entries, at_diag, lower, upper, split, nw, limits)
@@ -702,17 +721,15 @@ def level_programs(mech: dict, split: bool, nw: int):
             for k in (1, 2, 3):
                 if f[k] < n:
                     rest = [x for q, x in enumerate(f) if q not in (0, k)]
-                    by_species[f[k]].append(8 * j | 8 * len(apart) << 16)
+                    by_species[f[k]].append(_pack(8 * j, 8 * len(apart)))
                     apart.append([f[0]] + rest + [one_x])
         react = [[] for _ in range(nreact)]
         for i, j, v in mech["stoich"]:
-            react[j].append(8 * slot(scoef, float(codegen.literal(v))) | 8 * i << 16)
-        if 8 * len(apart) >= 1 << 16:
-            return None
+            react[j].append(_pack(8 * slot(scoef, float(codegen.literal(v))), 8 * i))
         segs["sweept"] = best["sweept"]
-        segs["tj"] = Segment(nw, 8 * n << 16).sums([((8 * j, 0), w) for j, w in enumerate(react)], True)
+        segs["tj"] = Segment(nw, _pack(0, 8 * n)).sums([((8 * j, 0), w) for j, w in enumerate(react)], True)
         segs["apart"] = Segment(nw, no_rate, None).rates([words4(f) for f in apart])
-        segs["vthl"] = Segment(nw, 8 * nreact | 8 * len(apart) << 16).sums(
+        segs["vthl"] = Segment(nw, _pack(8 * nreact, 8 * len(apart))).sums(
             [((8 * i, 0), w) for i, w in enumerate(by_species)], True)
     return {"segs": segs, "parts": len(parts), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
             "nbp": [len(part) for part in parts], "ng": best["ng"], "place": best["place"], "tail": tail,
@@ -738,6 +755,8 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
     the sweeps' one, for one choice of parts; estimate: only their cost, the
     factorisation's from the products per level."""
     t0 = n - tail
+    if 2 * n + 2 >= 1 << 16:
+        raise Unsupported("vector of the sweeps beyond 16-bit indices")
     fwd, bwd = ([], []) if limits is None else \
         (_parts(t0, lower, range(t0), limits[0]), _parts(t0, upper, range(t0 - 1, -1, -1), limits[1]))
     at = {}                                # (row, column) -> index of V or T
@@ -748,6 +767,8 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
                     at[(i, j)] = block + tail * tail + len(at)
     rbase = block + tail * tail + len(at)    # -R, then -1, then 0
     minus, zero = rbase + n, rbase + n + 1
+    if zero >= 1 << 16 and not estimate:
+        raise Unsupported("factors beyond 16-bit indices")
     # nodes: index, start value read, scale, flags, products
     level, nodes = {minus: 0}, []
 
