@@ -47,7 +47,7 @@
 #include <float.h>
 #include <limits.h>
 #include "rodas3_device.cuh"
-#include "gc_pow.h"
+#include "gc_root.h"
 #include "rodas3_kernels.h"
 /* sums may be split over lanes where the build need not round like the
    reference */
@@ -658,21 +658,10 @@ __device__ __forceinline__ int coop_end(CoopCell& c, const CoopArgs& a, double* 
   return 1;
 }
 
-/* err**(1/3) of the step-size factor.  gc_pow's double-double series is a
-   chain of ~1,000 dependent operations, a fifth of an attempt here.  The
-   production build starts from cbrt and adds the residual of one
-   double-double cube and the difference between the double 1/3 and 1/3
-   (x**(1/3 - d) = x**(1/3) (1 - d ln x), d = 1.850371707708594e-17); the one
-   rounding left is the last addition, as in gc_pow. */
+/* err**(1/3) of the step-size factor */
 __device__ __forceinline__ double coop_root(double x) {
 #if COOP_SPLIT
-  if (x < 1.0e300) {
-    const double c = cbrt(x);
-    const double p = c * c, pl = __fma_rn(c, c, -p);
-    const double q = p * c, ql = __fma_rn(p, c, -q) + pl * c;
-    const double r = (x - q) - ql;
-    return c + (r / (3.0 * p) - c * (1.850371707708594e-17 * log(x)));
-  }
+  if (x < 1.0e300) return gc_root3(x);
 #endif
   return gc_pow(x, 1.0 / ROS_ELO);
 }
