@@ -515,10 +515,11 @@ def _programs(mech, split, nw):
     def slot(table, value):
         return table.setdefault(value, len(table))
 
-    def product(node):
+    def product(node, sign=1.0):
         """[first, f1, f2, f3]: first indexes [RCT | extra], the others
         [V | FIX | ext]; missing factors are the constant 1, whose product
-        is exact.  A leading RCT(j)*literal is formed once per cell."""
+        is exact.  A leading RCT(j)*literal is formed once per cell.  A
+        negative sign goes into the first factor, which rounds alike."""
         fs = []
         while isinstance(node, list) and node[0] == "*":
             fs.append(node[2])
@@ -540,13 +541,13 @@ def _programs(mech, split, nw):
 
         f0 = fs[0]
         if f0[0] == "k" and len(fs) > 1 and fs[1][0] == "n":
-            first, fs = nreact + slot(extra, (f0[1], num(fs[1]))), fs[1:]
+            first, fs = nreact + slot(extra, (f0[1], sign * num(fs[1]))), fs[1:]
         elif f0[0] == "k":
-            first = f0[1]
+            first = f0[1] if sign > 0 else nreact + slot(extra, (f0[1], sign))
         elif f0[0] == "n":
-            first = nreact + slot(extra, (-1, num(f0)))
+            first = nreact + slot(extra, (-1, sign * num(f0)))
         else:                  # 1*v is exact
-            first, fs = nreact + slot(extra, (-1, 1.0)), [None] + fs
+            first, fs = nreact + slot(extra, (-1, sign)), [None] + fs
         rest = [other(f) for f in fs[1:]]
         if len(rest) > 3:
             raise Unsupported("product of more than four factors")
@@ -605,10 +606,7 @@ def _programs(mech, split, nw):
             for sign, t in signed(e):
                 if t[0] == "n" and float(codegen.literal(t[1])) == 0.0 and not words:
                     continue
-                f = product(t)
-                if sign < 0 or f[3] != n + nfix:
-                    raise Unsupported("destruction term")
-                words.append(f)
+                words.append(product(t, sign))
             dest.append((i, words))
         prod = [(i, scaled(e, "a", lambda j: j)) for i, e in enumerate(mech["prod"])]
         jvs = [scaled(e, "b", lambda j: bmap[j], -1.0) for e in mech["jvs"]]
@@ -629,8 +627,9 @@ def _programs(mech, split, nw):
     no_rate, no_sum = (_pack(zero, one), _pack(one, one)), _pack(0, 8 * nreact)
     segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
             "dest": None, "bufd": None, "prod": None, "bufp": None}
-    # a destruction term of three factors has no place in a line's words
-    long_d = [i for i, w in dest if len(w) > LONG and split or any(f[2] != n + nfix and f[1] != n + nfix for f in w)]
+    # a destruction term of three factors or more has no place in a line's words
+    long_d = [i for i, w in dest if len(w) > LONG and split or
+              any(sum(x != n + nfix for x in f[1:]) > 1 for f in w)]
     long_p = [i for i, w in prod if len(w) > LONG and split or i in long_d]
     if len(long_p) > 32:
         raise Unsupported("more than 32 long sums")
@@ -651,7 +650,7 @@ def _programs(mech, split, nw):
     if not long_p:
         del segs["bufd"], segs["bufp"]
     segs["dest"] = Segment(nw, _pack(zero, one)).lines(
-        [((8 * i, 0), [_pack(8 * f[0], 8 * (f[1] if f[2] == n + nfix else f[2])) for f in w])
+        [((8 * i, 0), [_pack(8 * f[0], 8 * next((x for x in f[1:] if x != n + nfix), n + nfix)) for f in w])
          for i, w in dest if i not in long_d])
     if long_p:
         segs["bufd"] = Segment(nw, no_rate, None).rates(rates_d)

@@ -44,3 +44,23 @@ def test_offsets_beyond_16_bits_do_not_corrupt(nreact):
     more than 8,192 places."""
     m = mechanism(30, nreact)
     agrees(m, True, 4)
+
+
+def with_dest(m, terms):
+    """The mechanism with other destruction sums for its first species."""
+    return dict(m, dest=[e if e is not None else d for e, d in
+                         zip(list(terms) + [None] * (m["nvar"] - len(terms)), m["dest"])])
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_destruction_sums_of_every_form(split):
+    """Negative terms, with and without literals, and products of four factors."""
+    m = mechanism(24, 90)
+    k, v, num, mul = (lambda j: ["k", j]), (lambda i: ["v", i]), (lambda x: ["n", x]), (lambda a, b: ["*", a, b])
+    m = with_dest(m, [
+        ["-", ["+", k(0), mul(k(1), v(2))], mul(k(3), v(4))],
+        ["+", ["neg", mul(mul(k(5), num("2")), v(1))], k(6)],
+        ["-", mul(mul(mul(k(7), v(3)), v(4)), v(5)), mul(num("3"), v(6))],
+        ["-", ["neg", v(7)], mul(mul(k(8), num("0.5")), v(9))],
+    ])
+    assert agrees(m, split, 4)
