@@ -580,23 +580,22 @@ def _programs(mech, split, nw):
 
     try:
         rate = [product(e) for e in mech["rates"]]
-        # partials B: each feeds one column of the Jacobian only, so they are
-        # formed for a part of the columns at a time, as many as the rates'
-        # scratch array holds
-        col_of = {}
+        # partials B are formed for a part of the columns at a time, as many as
+        # the rates' scratch array holds; each feeds one column of the Jacobian
+        # as KPP writes them, one read by several is formed for each
+        column = [set() for _ in range(n)]
         for p, e in enumerate(mech["jvs"]):
-            for b in codegen._refs(e, "b"):
-                if col_of.setdefault(b, icol[p]) != icol[p]:
-                    raise Unsupported("partial of two columns")
-        bexpr = dict(mech["jac_b"])
-        parts, part_of = [[]], {}
+            column[icol[p]].update(codegen._refs(e, "b"))
+        bexpr = dict.fromkeys(range(mech["nb"]), ["n", "0"])
+        bexpr.update(mech["jac_b"])
+        parts, part_of, bmap = [[]], {}, {}
         for c in range(n):
-            mine = sorted(b for b, k in col_of.items() if k == c)
-            if len(parts[-1]) + len(mine) > nreact:
+            if len(parts[-1]) + len(column[c]) > nreact:
                 parts.append([])
             part_of[c] = len(parts) - 1
-            parts[-1] += mine
-        bmap = {b: k for part in parts for k, b in enumerate(part)}
+            for b in sorted(column[c]):
+                bmap[(b, c)] = len(parts[-1])
+                parts[-1].append(b)
         if max(len(part) for part in parts) > nreact:
             raise Unsupported("column with too many partials")
         bpart = [[product(bexpr[b]) for b in part] for part in parts]
@@ -609,7 +608,7 @@ def _programs(mech, split, nw):
                 words.append(product(t, sign))
             dest.append((i, words))
         prod = [(i, scaled(e, "a", lambda j: j)) for i, e in enumerate(mech["prod"])]
-        jvs = [scaled(e, "b", lambda j: bmap[j], -1.0) for e in mech["jvs"]]
+        jvs = [scaled(e, "b", lambda j, c=c: bmap[(j, c)], -1.0) for e, c in zip(mech["jvs"], icol)]
     except KeyError as e:
         raise Unsupported(f"missing partial {e}") from None
     nx = n + nfix + len(ext)

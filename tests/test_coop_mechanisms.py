@@ -64,3 +64,17 @@ def test_destruction_sums_of_every_form(split):
         ["-", ["neg", v(7)], mul(mul(k(8), num("0.5")), v(9))],
     ])
     assert agrees(m, split, 4)
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_partial_of_several_columns(split):
+    """An entry that reads a partial of another column."""
+    m = mechanism(24, 90)
+    jvs, icol = list(m["jvs"]), m["lu_icol"]
+    first = next(p for p, e in enumerate(jvs) if codegen._refs(e, "b"))
+    b = codegen._refs(jvs[first], "b")[0]
+    others = [p for p in range(m["nnz"]) if icol[p] != icol[first] and codegen._refs(jvs[p], "b")]
+    for p in others[:3]:
+        jvs[p] = ["+", jvs[p], ["b", b]]
+    jvs[others[3]] = ["-", jvs[others[3]], ["*", ["n", "2"], ["b", b]]]
+    assert agrees(dict(m, jvs=jvs), split, 4)
