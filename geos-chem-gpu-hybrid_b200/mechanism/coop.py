@@ -670,7 +670,7 @@ def _programs(mech, split, nw):
             for jj in range(diag[j] + 1, crow[j + 1]):
                 upd[where[(i, icol[jj])]].append((kk, jj))
     # the tail block: its entries live in a dense array behind G
-    tail = _tail_rows(n, row_of, icol) if split else 0
+    tail = _tail_rows(n, row_of, icol, nreact) if split else 0
     t0 = n - tail
     in_tail = [row_of[p] >= t0 and icol[p] >= t0 for p in range(nnz)]
     block = nnz - sum(in_tail)
@@ -680,7 +680,7 @@ def _programs(mech, split, nw):
     for p in range(nnz):
         if in_tail[p]:
             place[p] = block + (row_of[p] - t0) * tail + icol[p] - t0
-    if 2 * tail > nreact or 8 * (block + tail * tail) > NO_ENTRY:
+    if 8 * (block + tail * tail) > NO_ENTRY:
         raise Unsupported("tail block")
     # -Jac0 (the coefficients carry the sign); the kernel adds ghinv to the
     # diagonal and forms the reciprocals of the diagonals without updates
@@ -740,10 +740,11 @@ def _programs(mech, split, nw):
 INVERSE_LIMITS = (0, 50, 100, 200, 400)
 
 
-def _tail_rows(n, row_of, icol):
-    """Rows of the tail block: 64 where they are dense, else 32."""
+def _tail_rows(n, row_of, icol, nreact):
+    """Rows of the tail block: 64 where they are dense, else 32; the rates'
+    scratch array hands over two of them at a time."""
     for m, least in ((64, 0.9), (32, 0.0)):
-        if n >= 2 * m - 8 and sum(r >= n - m and c >= n - m for r, c in zip(row_of, icol)) >= least * m * m:
+        if n >= 2 * m - 8 and nreact >= 2 * m and sum(r >= n - m and c >= n - m for r, c in zip(row_of, icol)) >= least * m * m:
             return m
     return 0
 

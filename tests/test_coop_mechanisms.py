@@ -78,3 +78,12 @@ def test_partial_of_several_columns(split):
         jvs[p] = ["+", jvs[p], ["b", b]]
     jvs[others[3]] = ["-", jvs[others[3]], ["*", ["n", "2"], ["b", b]]]
     assert agrees(dict(m, jvs=jvs), split, 4)
+
+
+@pytest.mark.parametrize("nreact,tail", [(63, 0), (64, 32)])
+def test_fewer_rates_than_two_tail_rows(nreact, tail):
+    """The tail block's elimination hands its pivot rows over in the rates'
+    scratch array; a mechanism with fewer rates goes without the block."""
+    m = mechanism(60, nreact)
+    assert agrees(m, True, 4)
+    assert coop.level_programs(m, True, 4)["tail"] == tail
