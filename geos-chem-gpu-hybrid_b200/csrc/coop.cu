@@ -404,8 +404,8 @@ __device__ __forceinline__ void coop_run(unsigned int cell, CoopFetch& f, int se
   }
 }
 
-/* Fun's long sums (a lane per sum, chains[32] = species, first product, blocks):
-   the products wait in B, so a term costs a load and an addition, in order. */
+/* Fun's long sums (a lane per sum: species, first product, blocks): the
+   products wait in B, so a term costs a load and an addition, in order. */
 template <int NT>
 __device__ __forceinline__ double coop_chain(const double* sm, int first, int blocks) {
   const double2* b = reinterpret_cast<const double2*>(sm + CoopAt<NT>::B + first);
@@ -492,12 +492,27 @@ __device__ __forceinline__ void coop_tail(double* sm) {
 }
 #endif
 
-/* a thread's long sum: the first warp's are productions, the last's destructions */
+/* a thread's long sum of round r (32 sums each): the first warp's are
+   productions, the last's destructions */
 template <int NT>
-__device__ __forceinline__ void coop_chain_load(int* chain) {
-  const int tid = threadIdx.x % NT, k = 3 * (tid & 31) + (tid < 32 ? 96 : 0);
+__device__ __forceinline__ void coop_chain_load(int* chain, int r = 0) {
+  const int tid = threadIdx.x % NT, k = 3 * (32 * r + (tid & 31) + (tid < 32 ? 32 * COOP_CHAINS : 0));
 #pragma unroll
   for (int t = 0; t < 3; ++t) chain[t] = coop_chain_of[k + t];
+}
+
+/* the warp's long sums, finish(species, sum); the first round's are kept in
+   registers over the solve (`chain`), further ones are rare */
+template <int NT, class F>
+__device__ __forceinline__ void coop_chains(const double* sm, const int* chain, F finish) {
+  int c[3] = {chain[0], chain[1], chain[2]};
+#pragma unroll 1
+  for (int r = 0;;) {
+    const double x = coop_chain<NT>(sm, c[1], c[2]);
+    if (c[0] >= 0) finish(c[0], x);
+    if (++r == COOP_CHAINS) break;
+    coop_chain_load<NT>(c, r);
+  }
 }
 
 /* Fun_SPLIT of the state in V into X; `after`: the segment that follows */
@@ -516,18 +531,13 @@ __device__ __forceinline__ void coop_fun(unsigned int cell, CoopFetch& f, double
   coop_sync<NT, NG>();
   /* the last warp adds up the long destruction sums, then the first the
      long production sums, which wait for all products */
-  if (tid >= NT - 32) {
-    const double d = coop_chain<NT>(sm, chain[1], chain[2]);
-    if (chain[0] >= 0) sm[L::X + chain[0]] = d;
-  }
+  if (tid >= NT - 32)
+    coop_chains<NT>(sm, chain, [sm](int i, double d) { sm[L::X + i] = d; });
   coop_run<P_PROD, NT, NG>(cell, f, COOP_SEG_PROD, COOP_SEG_BUFP);
   coop_run<P_BUFP, NT, NG>(cell, f, COOP_SEG_BUFP, after);
   coop_sync<NT, NG>();
-  if (tid < 32) {
-    const int i = chain[0];
-    const double p = coop_chain<NT>(sm, chain[1], chain[2]);
-    if (i >= 0) sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i];
-  }
+  if (tid < 32)
+    coop_chains<NT>(sm, chain, [sm](int i, double p) { sm[L::X + i] = p - sm[L::X + i] * sm[L::V + i]; });
 #else
   coop_run<P_DEST, NT, NG>(cell, f, COOP_SEG_DEST, COOP_SEG_PROD);
   coop_sync<NT, NG>();

@@ -630,8 +630,6 @@ def _programs(mech, split, nw):
     long_d = [i for i, w in dest if len(w) > LONG and split or
               any(sum(x != n + nfix for x in f[1:]) > 1 for f in w)]
     long_p = [i for i, w in prod if len(w) > LONG and split or i in long_d]
-    if len(long_p) > 32:
-        raise Unsupported("more than 32 long sums")
     # the buffer: the long sums' products, each sum padded to whole blocks
     first = {}
 
@@ -657,7 +655,7 @@ def _programs(mech, split, nw):
     if long_p:
         segs["bufp"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(
             [(8 * (len(rates_d) + k), w) for k, w in enumerate(ones_p)])
-    # lane l's chain: species, first product, blocks
+    # chain l of lane l % 32: species, first product, blocks
     chains = [[(i,) + first[(key, i)] for i in rows] for key, rows in (("d", long_d), ("p", long_p))]
     # KppDecomp entry by entry: G(i,c) = G(i,c) - sum L(i,j) U(j,c), and for
     # c < i the product with 1/U(c,c); an entry's level is one above those of
@@ -942,6 +940,7 @@ def coop_inc(mech: dict) -> str:
         lines.append("#if COOP_SPLIT" if split else "#if !COOP_SPLIT")
         for nw in (4, 8):
             p = level_programs(mech, split, nw)
+            rounds = max([1] + [-(-len(c) // 32) for c in p["chains"]])
             if nw == 4:
                 lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
                           f"#define COOP_NEXTRA {len(p['extra'])}", f"#define COOP_PARTS {p['parts']}",
@@ -953,7 +952,8 @@ def coop_inc(mech: dict) -> str:
                           f"#define COOP_NAPART {p['napart']}", f"#define COOP_NSCOEF {len(p['scoef'])}",
                           doubles("coop_scoef", p["scoef"]), arr("unsigned char", "coop_has_k", p["has_k"]),
                           f"#define COOP_BUFFER {p['buffer']}", f"#define COOP_NBUFD {p['nbufd']}",
-                          arr("int", "coop_chain_of", [x for c in p["chains"] for k in range(32)
+                          f"#define COOP_CHAINS {rounds}",
+                          arr("int", "coop_chain_of", [x for c in p["chains"] for k in range(32 * rounds)
                                                     for x in (c[k] if k < len(c) else (-1, 0, 0))]),
                           f"#define COOP_TAIL {p['tail']}", f"#define COOP_BLOCK {p['block']}", "#define COOP_NBP(q) (%s)" % " : ".join(
                               [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),

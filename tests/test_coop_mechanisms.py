@@ -87,3 +87,13 @@ def test_fewer_rates_than_two_tail_rows(nreact, tail):
     m = mechanism(60, nreact)
     assert agrees(m, True, 4)
     assert coop.level_programs(m, True, 4)["tail"] == tail
+
+
+def test_more_long_sums_than_lanes():
+    """40 species in 1,400 reactions: production sums of more than 60 terms take
+    two rounds of a warp's lanes."""
+    m = mechanism(40, 1400)
+    assert agrees(m, True, 4)
+    p = coop.level_programs(m, True, 4)
+    assert len(p["chains"][1]) > 32
+    assert "#define COOP_CHAINS 2" in coop.coop_inc(m)
