@@ -79,6 +79,12 @@ struct CoopAt {
   static constexpr int CELL = (RED + 10) / 2 * 2;
 };
 extern __shared__ __align__(16) unsigned char coop_smem[];
+/* the generator fits the cell into shared memory by the same sum */
+static_assert(CoopAt<128>::CELL == COOP_CELL4 && CoopAt<256>::CELL == COOP_CELL8, "layout of a cell");
+/* offsets in the streams: bytes (COOP_UNIT 8), or doubles where an array is
+   beyond the 64 KB that 16 bits reach (COOP_UNIT 1; then a multiplication more
+   for each).  An element's offset is its index times COOP_UNIT. */
+#define COOP_BYTES (8 / COOP_UNIT)
 
 /* control bits of the streams (mechanism/coop.py) */
 #define CL_LEAD   1u
@@ -170,21 +176,21 @@ __device__ __forceinline__ void coop_sync(void) {
 }
 
 /* Shared-memory access by 32-bit address: `cell` is the address of the cell's
-   first array, SO a compile-time place, off a byte offset from a stream. */
+   first array, SO a compile-time place, off an offset from a stream. */
 template <int SO>
 __device__ __forceinline__ double coop_get(unsigned int cell, unsigned int off) {
   double x;
-  asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(x) : "r"(cell + off), "n"(SO * 8));
+  asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(x) : "r"(cell + off * COOP_BYTES), "n"(SO * 8));
   return x;
 }
 template <int SO>
 __device__ __forceinline__ void coop_put(unsigned int cell, unsigned int off, double x) {
-  asm volatile("st.shared.f64 [%0+%1], %2;" :: "r"(cell + off), "n"(SO * 8), "d"(x) : "memory");
+  asm volatile("st.shared.f64 [%0+%1], %2;" :: "r"(cell + off * COOP_BYTES), "n"(SO * 8), "d"(x) : "memory");
 }
 template <int SO>
 __device__ __forceinline__ void coop_put_if(bool p, unsigned int cell, unsigned int off, double x) {
   asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q st.shared.f64 [%0+%1], %2; }"
-               :: "r"(cell + off), "n"(SO * 8), "d"(x), "r"((unsigned int)p) : "memory");
+               :: "r"(cell + off * COOP_BYTES), "n"(SO * 8), "d"(x), "r"((unsigned int)p) : "memory");
 }
 
 /* a word that all lanes of the warp hold, as a warp-uniform value: branches on
@@ -237,7 +243,7 @@ __device__ __forceinline__ void coop_rate_op(unsigned int cell, uint4 a, uint4 b
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    coop_put_if<OUT>(j + k * step < n, cell, 8 * (j + k * step),
+    coop_put_if<OUT>(j + k * step < n, cell, COOP_UNIT * (j + k * step),
                       ((f[k][0] * f[k][1]) * f[k][2]) * f[k][3]);
 }
 
@@ -321,7 +327,7 @@ __device__ __forceinline__ double coop_level_op(unsigned int cell, double acc, u
   if (u & CL_FIRST) {
     acc = 0.0;
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.shared.f64 %0, [%1+%3]; }"
-                 : "+d"(acc) : "r"(cell + d), "r"(ctl & CL_START), "n"(BASE * 8));
+                 : "+d"(acc) : "r"(cell + d * COOP_BYTES), "r"(ctl & CL_START), "n"(BASE * 8));
   }
   if (u & (4u << 12)) {                    /* more than three products */
 #pragma unroll

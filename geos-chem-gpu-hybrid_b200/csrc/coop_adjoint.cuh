@@ -81,7 +81,7 @@ __device__ __forceinline__ void adj_dual_op(unsigned int cell, uint4 a, uint4 b,
     const unsigned int o0 = w[2 * k] & 0xFFFFu, o1 = w[2 * k] >> 16, o2 = w[2 * k + 1] & 0xFFFFu;
     const double z1 = coop_get<L::YB>(cell, o1), z2 = coop_get<L::YB>(cell, o2);
     const double k1 = coop_get<L::KX>(cell, o1), k2 = coop_get<L::KX>(cell, o2);
-    coop_put_if<L::DM>(j + k * 128 < COOP_NAPART, cell, 8 * (j + k * 128),
+    coop_put_if<L::DM>(j + k * 128 < COOP_NAPART, cell, COOP_UNIT * (j + k * 128),
                        coop_get<L::RX>(cell, o0) * (k1 * z2 + z1 * k2));
   }
 }
@@ -103,9 +103,9 @@ __device__ __forceinline__ void adj_mu_op(unsigned int cell, uint4 a, uint4 b, i
       const double ka = coop_get<L::KX>(cell, o[0]), kb = coop_get<L::KX>(cell, o[1]),
                    kc = coop_get<L::KX>(cell, o[2]);
       const double dak = c * (ka * zb * zc + kb * za * zc + kc * za * zb);
-      const double x = coop_get<L::MU>(cell, 8 * j) +
-                       coop_get<L::T>(cell, 8 * j) * (((c * ea) * eb) * ec + dak);
-      coop_put<L::MU>(cell, 8 * j, x);
+      const double x = coop_get<L::MU>(cell, COOP_UNIT * j) +
+                       coop_get<L::T>(cell, COOP_UNIT * j) * (((c * ea) * eb) * ec + dak);
+      coop_put<L::MU>(cell, COOP_UNIT * j, x);
     }
   }
 }

@@ -227,8 +227,9 @@ def compile_tables(mech: dict):
 # the kernel fetches operations several ahead of their use.
 #
 # Operands are given as byte offsets in their array (the kernel keeps the cell
-# in shared memory), so that a word needs no arithmetic; a missing operand
-# points at a constant 0 (or 1) behind the array, so that it needs no test.
+# in shared memory), so that a word needs no arithmetic, or, in a mechanism whose
+# arrays are beyond 64 KB, as indices that the kernel multiplies (COOP_UNIT); a
+# missing operand points at a constant 0 (or 1) behind the array, so that it needs no test.
 #
 #   rate operations   four products (f0 | f1<<16, f2 | f3<<16).  Product k of
 #                     operation i of warp w and lane l is number
@@ -435,10 +436,10 @@ class Segment:
                     self.ops[v].append([[h, c | diags] + w for h, c, w in op])
         self._sync()
 
-    def in_bytes(self):
+    def in_units(self, unit):
         """Element indices (both halves of headers and words) as offsets."""
         def offsets(w):
-            return _pack(8 * (w & 0xFFFF), 8 * (w >> 16))
+            return _pack(unit * (w & 0xFFFF), unit * (w >> 16))
 
         for ops in self.ops:
             for op in ops:
@@ -490,23 +491,45 @@ def _parts(n, deps, order, limit):
     return out
 
 
+SHARED = 227 * 1024 // 8    # doubles of shared memory that a block may have
+
+
+def cell_doubles(ng, nx, n, nreact, nextra, buffer):
+    """Shared memory of a cell (CoopAt in csrc/coop.cu)."""
+    products = (ng + 1 + nx + 2 * n + 2 + nreact + 1 + nreact + nextra + 2) // 2 * 2
+    return (products + buffer + 10) // 2 * 2
+
+
 def level_programs(mech: dict, split: bool, nw: int):
     """The cooperative kernel's programs, or None for expression shapes or
     sizes that they do not hold.  split: sums may be divided over lanes
     (production build); nw: warps of the block."""
     try:
-        return _programs(mech, split, nw)
+        return _fitting_programs(mech, split, nw)
     except Unsupported:
         return None
 
 
-def _programs(mech, split, nw):
+def _fitting_programs(mech, split, nw):
+    """Offsets are in bytes where 16 bits hold them, else in doubles ("unit").
+    A cell that does not fit in shared memory goes without the buffer of the
+    long sums, then without the tail block; the inverses of the sweeps' parts
+    are chosen within what is left.  What is taken does not depend on nw."""
+    why = None
+    for long, with_tail in ((LONG, True), (1 << 30, True), (1 << 30, False)):
+        for unit in (8, 1):
+            try:
+                return _programs(mech, split, nw, unit, long, with_tail)
+            except Unsupported as e:
+                why = why or e
+    raise why
+
+
+def _programs(mech, split, nw, unit, long, with_tail):
     if compile_tables(mech) is None:
         raise Unsupported("expression shape")
     n, nfix, nnz, nreact = mech["nvar"], mech["nfix"], mech["nnz"], mech["nreact"]
     crow, diag, icol, where = mech["lu_crow"], mech["lu_diag"], mech["lu_icol"], mech["lu_where"]
-    if 8 * nnz >= 1 << 16:
-        raise Unsupported("factors beyond 16-bit offsets")
     extra = {}                 # first factors behind the rate constants: (reaction or
                                # -1, literal), the literal itself or RCT(j)*literal
     ext = {1.0: 0}             # constants behind the species (other factors)
@@ -612,24 +635,22 @@ def _programs(mech, split, nw):
     except KeyError as e:
         raise Unsupported(f"missing partial {e}") from None
     nx = n + nfix + len(ext)
-    zero = 8 * (nreact + len(extra))     # the constant 0 behind [RCT | extra]
-    one = 8 * (n + nfix)
-    if max(8 * nx, zero, 8 * len(coef)) >= 1 << 16:
-        raise Unsupported("vectors beyond 16-bit offsets")
+    zero = unit * (nreact + len(extra))  # the constant 0 behind [RCT | extra]
+    one = unit * (n + nfix)
 
     def words4(f):
-        return [_pack(8 * f[0], 8 * f[1]), _pack(8 * f[2], 8 * f[3])]
+        return [_pack(unit * f[0], unit * f[1]), _pack(unit * f[2], unit * f[3])]
 
     def scaled_words(words):
-        return [_pack(8 * (w & 0xFFFF), 8 * (w >> 16)) for w in words]
+        return [_pack(unit * (w & 0xFFFF), unit * (w >> 16)) for w in words]
 
-    no_rate, no_sum = (_pack(zero, one), _pack(one, one)), _pack(0, 8 * nreact)
+    no_rate, no_sum = (_pack(zero, one), _pack(one, one)), _pack(0, unit * nreact)
     segs = {"rate": Segment(nw, no_rate, None).rates([words4(f) for f in rate]),
             "dest": None, "bufd": None, "prod": None, "bufp": None}
     # a destruction term of three factors or more has no place in a line's words
-    long_d = [i for i, w in dest if len(w) > LONG and split or
+    long_d = [i for i, w in dest if len(w) > long and split or
               any(sum(x != n + nfix for x in f[1:]) > 1 for f in w)]
-    long_p = [i for i, w in prod if len(w) > LONG and split or i in long_d]
+    long_p = [i for i, w in prod if len(w) > long and split or i in long_d]
     # the buffer: the long sums' products, each sum padded to whole blocks
     first = {}
 
@@ -647,14 +668,14 @@ def _programs(mech, split, nw):
     if not long_p:
         del segs["bufd"], segs["bufp"]
     segs["dest"] = Segment(nw, _pack(zero, one)).lines(
-        [((8 * i, 0), [_pack(8 * f[0], 8 * next((x for x in f[1:] if x != n + nfix), n + nfix)) for f in w])
+        [((unit * i, 0), [_pack(unit * f[0], unit * next((x for x in f[1:] if x != n + nfix), n + nfix)) for f in w])
          for i, w in dest if i not in long_d])
     if long_p:
         segs["bufd"] = Segment(nw, no_rate, None).rates(rates_d)
-    segs["prod"] = Segment(nw, no_sum).lines([((8 * i, 0), scaled_words(w)) for i, w in prod if i not in long_p])
+    segs["prod"] = Segment(nw, no_sum).lines([((unit * i, 0), scaled_words(w)) for i, w in prod if i not in long_p])
     if long_p:
-        segs["bufp"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(
-            [(8 * (len(rates_d) + k), w) for k, w in enumerate(ones_p)])
+        segs["bufp"] = Segment(nw, (NO_ENTRY, unit * nreact), None).singles(
+            [(unit * (len(rates_d) + k), w) for k, w in enumerate(ones_p)])
     # chain l of lane l % 32: species, first product, blocks
     chains = [[(i,) + first[(key, i)] for i in rows] for key, rows in (("d", long_d), ("p", long_p))]
     # KppDecomp entry by entry: G(i,c) = G(i,c) - sum L(i,j) U(j,c), and for
@@ -668,7 +689,7 @@ def _programs(mech, split, nw):
             for jj in range(diag[j] + 1, crow[j + 1]):
                 upd[where[(i, icol[jj])]].append((kk, jj))
     # the tail block: its entries live in a dense array behind G
-    tail = _tail_rows(n, row_of, icol, nreact) if split else 0
+    tail = _tail_rows(n, row_of, icol, nreact) if split and with_tail else 0
     t0 = n - tail
     in_tail = [row_of[p] >= t0 and icol[p] >= t0 for p in range(nnz)]
     block = nnz - sum(in_tail)
@@ -678,14 +699,14 @@ def _programs(mech, split, nw):
     for p in range(nnz):
         if in_tail[p]:
             place[p] = block + (row_of[p] - t0) * tail + icol[p] - t0
-    if 8 * (block + tail * tail) > NO_ENTRY:
+    if unit * (block + tail * tail) > NO_ENTRY:
         raise Unsupported("tail block")
     # -Jac0 (the coefficients carry the sign); the kernel adds ghinv to the
     # diagonal and forms the reciprocals of the diagonals without updates
     fill = set(range(block, block + tail * tail)) - {place[p] for p in range(nnz)}
     for q, part in enumerate(bpart):
-        mine = [(8 * place[p], scaled_words(jvs[p])) for p in range(nnz) if part_of[icol[p]] == q]
-        mine += [(8 * p, []) for p in sorted(fill)] if q == 0 else []
+        mine = [(unit * place[p], scaled_words(jvs[p])) for p in range(nnz) if part_of[icol[p]] == q]
+        mine += [(unit * p, []) for p in sorted(fill)] if q == 0 else []
         segs[f"bpart{q}"] = Segment(nw, no_rate, None).rates([words4(f) for f in part])
         segs[f"jvs{q}"] = Segment(nw, no_sum).sums([((h, 0), w) for h, w in mine if len(w) > 1], split)
         segs[f"one{q}"] = [(h, w[0] if w else no_sum) for h, w in mine if len(w) <= 1]
@@ -695,19 +716,29 @@ def _programs(mech, split, nw):
     entries = [(row_of[p], icol[p], place[p], [(place[a], place[b]) for a, b in upd[p] if icol[a] < t0])
                for p in range(nnz)]
     at_diag = [place[p] for p in diag]
+    buffered = len(rates_d) + len(ones_p)
+    coefs = len(coef) + len(coef) % 2
+
+    def fits(ng):
+        return unit * ng < 1 << 16 and coefs + cell_doubles(ng, nx, n, nreact, len(extra), buffered) <= SHARED
+
     limits = None
     if split:
         tried = [(f, u) for f in INVERSE_LIMITS for u in INVERSE_LIMITS]
-        # (the offsets of the factor array have to fit 16 bits)
-        tried = [lim for lim in tried if 8 * _factor_and_sweeps(
-            n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["ng"] < 1 << 16]
+        tried = [lim for lim in tried if fits(_factor_and_sweeps(
+            n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["ng"])]
         if not tried:
-            raise Unsupported("inverses beyond 16-bit offsets")
+            raise Unsupported("cell beyond 16-bit offsets or the shared memory of a block")
         limits = min(tried, key=lambda lim: _factor_and_sweeps(
             n, tail, block, entries, at_diag, lower, upper, split, nw, lim, True)["cost"])
     best = _factor_and_sweeps(n, tail, block, entries, at_diag, lower, upper, split, nw, limits)
+    if not fits(best["ng"]):
+        raise Unsupported("cell beyond 16-bit offsets or the shared memory of a block")
+    for f in ("lu", "sweep", "sweept"):
+        if f in best:
+            best[f].pad().in_units(unit)
     for q in range(len(bpart)):
-        segs[f"one{q}"] = Segment(nw, (NO_ENTRY, 8 * nreact), None).singles(segs[f"one{q}"])
+        segs[f"one{q}"] = Segment(nw, (NO_ENTRY, unit * nreact), None).singles(segs[f"one{q}"])
     segs["lu"], segs["sweep"] = best["lu"], best["sweep"]
     extra_of = [j for j, _ in extra]
     scoef, apart, by_species = {1.0: 0}, [], [[] for _ in range(n)]
@@ -717,19 +748,19 @@ def _programs(mech, split, nw):
             for k in (1, 2, 3):
                 if f[k] < n:
                     rest = [x for q, x in enumerate(f) if q not in (0, k)]
-                    by_species[f[k]].append(_pack(8 * j, 8 * len(apart)))
+                    by_species[f[k]].append(_pack(unit * j, unit * len(apart)))
                     apart.append([f[0]] + rest + [one_x])
         react = [[] for _ in range(nreact)]
         for i, j, v in mech["stoich"]:
-            react[j].append(_pack(8 * slot(scoef, float(codegen.literal(v))), 8 * i))
+            react[j].append(_pack(unit * slot(scoef, float(codegen.literal(v))), unit * i))
         segs["sweept"] = best["sweept"]
-        segs["tj"] = Segment(nw, _pack(0, 8 * n)).sums([((8 * j, 0), w) for j, w in enumerate(react)], True)
+        segs["tj"] = Segment(nw, _pack(0, unit * n)).sums([((unit * j, 0), w) for j, w in enumerate(react)], True)
         segs["apart"] = Segment(nw, no_rate, None).rates([words4(f) for f in apart])
-        segs["vthl"] = Segment(nw, _pack(8 * nreact, 8 * len(apart))).sums(
-            [((8 * i, 0), w) for i, w in enumerate(by_species)], True)
-    return {"segs": segs, "parts": len(parts), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
+        segs["vthl"] = Segment(nw, _pack(unit * nreact, unit * len(apart))).sums(
+            [((unit * i, 0), w) for i, w in enumerate(by_species)], True)
+    return {"segs": segs, "unit": unit, "parts": len(parts), "cell": cell_doubles(best["ng"], nx, n, nreact, len(extra), buffered), "extra": extra, "ext": ext, "coef": coef, "nx": nx,
             "nbp": [len(part) for part in parts], "ng": best["ng"], "place": best["place"], "tail": tail,
-            "chains": chains, "buffer": len(rates_d) + len(ones_p), "nbufd": len(rates_d), "factor": place, "block": block, "diag": [(at_diag[i], i < t0 and not upd[diag[i]]) for i in range(n)],
+            "chains": chains, "buffer": buffered, "nbufd": len(rates_d), "factor": place, "block": block, "diag": [(at_diag[i], i < t0 and not upd[diag[i]]) for i in range(n)],
             "cost": best["cost"], "scoef": scoef, "napart": len(apart), "place_t": best["place_t"],
             "has_k": [int(f[0] < nreact or extra_of[f[0] - nreact] >= 0) for f in rate]}
 
@@ -859,7 +890,6 @@ def _factor_and_sweeps(n, tail, block, entries, diag, lower, upper, split, nw, l
                           [block + (i - t0) * tail + j - t0 | x[j] << 16 for j in range(t0, n)])
                          for i in range(t0, n)], split, True)
             x = x[:t0] + new[t0:]
-    lu.pad().in_bytes(), sweep.pad().in_bytes()
     out = {"lu": lu, "sweep": sweep, "ng": zero, "place": x, "cost": lu.cost + 4 * sweep.cost}
     if limits is not None and not estimate:
         out["sweept"], out["place_t"] = _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw)
@@ -912,7 +942,7 @@ def _transposed(n, tail, block, fwd, bwd, lower, upper, at, rbase, split, nw):
             outside(range(t0, n), cols, lambda i: i < t0)
             product({j: [block + (i - t0) * tail + j - t0 | x[i] << 16 for i in range(t0, n)]
                      for j in range(t0, n)})
-    return seg.pad().in_bytes(), x
+    return seg, x
 
 
 EARLY = 2              # levels between an early product's readiness and its sum's end
@@ -922,10 +952,15 @@ def coop_inc(mech: dict) -> str:
     """coop.inc: MECH_COOP and, when the programs exist, their C arrays for
     both builds (COOP_SPLIT) and both block sizes, included by one translation
     unit."""
-    t = compile_tables(mech)
-    if t is None or level_programs(mech, True, 4) is None:
-        return "/* no cooperative-kernel tables: unsupported expression shape */\n" \
-               "#define MECH_COOP 0\n"
+    forms = {}
+    try:
+        for split in (False, True):
+            for nw in (4, 8):
+                forms[split, nw] = _fitting_programs(mech, split, nw)
+            for k in ("unit", "tail", "block", "buffer", "chains", "coef", "parts"):
+                assert forms[split, 4][k] == forms[split, 8][k], k
+    except Unsupported as e:
+        return f"/* no cooperative kernel for this mechanism: {e} */\n#define MECH_COOP 0\n"
 
     def arr(ctype, name, vals, space="__device__ const"):
         body = ",".join(str(v) for v in vals) if vals else "0"
@@ -935,11 +970,12 @@ def coop_inc(mech: dict) -> str:
         return arr("double", name, [repr(float(v)) for v in vals] or [0.0])
 
     lines = ["/* generated cooperative-kernel tables; do not edit */", "#pragma once",
-             "#define MECH_COOP 1", f"#define COOP_NUPD {len(t['upd'])}", f"#define COOP_DEPTH {DEPTH}"]
+             "#define MECH_COOP 1", f"#define COOP_NUPD {len(compile_tables(mech)['upd'])}",
+             f"#define COOP_DEPTH {DEPTH}"]
     for split in (False, True):
         lines.append("#if COOP_SPLIT" if split else "#if !COOP_SPLIT")
         for nw in (4, 8):
-            p = level_programs(mech, split, nw)
+            p = forms[split, nw]
             rounds = max([1] + [-(-len(c) // 32) for c in p["chains"]])
             if nw == 4:
                 lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
@@ -952,14 +988,15 @@ def coop_inc(mech: dict) -> str:
                           f"#define COOP_NAPART {p['napart']}", f"#define COOP_NSCOEF {len(p['scoef'])}",
                           doubles("coop_scoef", p["scoef"]), arr("unsigned char", "coop_has_k", p["has_k"]),
                           f"#define COOP_BUFFER {p['buffer']}", f"#define COOP_NBUFD {p['nbufd']}",
-                          f"#define COOP_CHAINS {rounds}",
+                          f"#define COOP_UNIT {p['unit']}", f"#define COOP_CHAINS {rounds}",
                           arr("int", "coop_chain_of", [x for c in p["chains"] for k in range(32 * rounds)
                                                     for x in (c[k] if k < len(c) else (-1, 0, 0))]),
                           f"#define COOP_TAIL {p['tail']}", f"#define COOP_BLOCK {p['block']}", "#define COOP_NBP(q) (%s)" % " : ".join(
                               [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),
                           arr("int", "coop_diag", [o << 1 | (e and 1) for o, e in p["diag"]])]
                 lines += [f"#define COOP_SEG_{name.upper()} {k}" for k, name in enumerate(p["segs"])]
-            lines += [arr("int", f"coop_place_t{nw}", p["place_t"]), f"#define COOP_NG{nw} {p['ng']}", arr("int", f"coop_place{nw}", p["place"])]
+            lines += [arr("int", f"coop_place_t{nw}", p["place_t"]), f"#define COOP_NG{nw} {p['ng']}",
+                      f"#define COOP_CELL{nw} {p['cell']}", arr("int", f"coop_place{nw}", p["place"])]
             words, where = [], []
             for seg in p["segs"].values():
                 for ops in seg.ops:

@@ -38,12 +38,36 @@ def test_shipped_mechanisms(name, split):
     assert agrees(codegen.load(name), split, 4)
 
 
-@pytest.mark.parametrize("nreact", [3000, 5000])
-def test_offsets_beyond_16_bits_do_not_corrupt(nreact):
-    """30 species in 3,000 and 5,000 reactions: the long sums' products need
-    more than 8,192 places."""
-    m = mechanism(30, nreact)
-    agrees(m, True, 4)
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("nspec,nreact,what", [(30, 3000, "buffer"), (135, 450, "factors")])
+def test_offsets_beyond_16_bits(nspec, nreact, what, split):
+    """30 species in 3,000 reactions: the long sums' products (production
+    build) need more than 8,192 places.  135 species in 450 reactions: 9,138
+    factors, 73 KB."""
+    m = mechanism(nspec, nreact)
+    assert agrees(m, split, 4)
+    p = coop.level_programs(m, split, 4)
+    wide = p["buffer"] > 8191 if what == "buffer" else p["ng"] > 8191
+    assert wide == (split or what == "factors")
+    assert p["unit"] == (1 if wide else 8)
+
+
+def test_cell_within_shared_memory():
+    """A cell that shared memory does not hold gets fewer inverses of the sweeps'
+    parts; one whose factors alone are too many gets no programs."""
+    m = mechanism(80, 200)
+    p = coop.level_programs(m, True, 4)
+    full = coop.SHARED
+    try:
+        coop.SHARED = p["cell"] + len(p["coef"]) - 200
+        q = coop.level_programs(m, True, 4)
+        assert q is not None and q["ng"] < p["ng"]
+        assert q["cell"] + len(q["coef"]) <= coop.SHARED
+        coop.SHARED = m["nnz"]
+        assert coop.level_programs(m, True, 4) is None
+        assert "shared memory" in coop.coop_inc(m)
+    finally:
+        coop.SHARED = full
 
 
 def with_dest(m, terms):
