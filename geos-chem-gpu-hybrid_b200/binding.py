@@ -23,6 +23,7 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_DIR = os.path.join(HERE, "lib")
 
+AUTO = -1           # cooperative or persistent, by the number of cells of a call
 PLAIN = 0
 PERSISTENT = 1
 PLAIN_FUSED = 2
@@ -251,8 +252,11 @@ class Solver:
             RCNTRL.data_ptr(), order.data_ptr(), ISTAT.data_ptr(),
             RSTAT.data_ptr(), IERR.data_ptr(), ctypes.c_void_p(stream.cuda_stream)))
 
-    def set_launch(self, mode: int = PERSISTENT, threads: int = 0,
+    def set_launch(self, mode: int = AUTO, threads: int = 0,
                    blocks_per_sm: int = 0) -> None:
+        """Kernel, block size and resident blocks of the calls that follow on
+        this device; ``AUTO``, the setting of a fresh process, chooses the
+        kernel by the number of cells."""
         if self.lib.gcchem_b200_set_launch(mode, threads, blocks_per_sm) != 0:
             raise ValueError("invalid launch settings")
 

@@ -7,7 +7,8 @@
 extern "C" {
 #endif
 
-enum { RODAS3_PLAIN = 0, RODAS3_PERSISTENT = 1, RODAS3_PLAIN_FUSED = 2, RODAS3_COOP = 3 };
+/* RODAS3_AUTO is a setting, resolved before a launch (auto_mode in gc_api.cu) */
+enum { RODAS3_AUTO = -1, RODAS3_PLAIN = 0, RODAS3_PERSISTENT = 1, RODAS3_PLAIN_FUSED = 2, RODAS3_COOP = 3 };
 
 typedef struct {
   int mode;              /* RODAS3_PLAIN, RODAS3_PERSISTENT, RODAS3_PLAIN_FUSED or RODAS3_COOP */

@@ -96,7 +96,10 @@ void gcchem_b200_sizes(int* nvar, int* nfix, int* nreact, int* nnz);
  * 3 = cooperative (one block of 128 or 256 threads per cell, the cell's
  * factors and vectors in shared memory, the same cost-ordered queue; no
  * solver workspace; for mechanisms whose state fits in shared memory --
- * gcchem_b200_set_launch returns -1 otherwise). */
+ * gcchem_b200_set_launch returns -1 otherwise).  -1 = automatic, the setting
+ * of a process that has named none: by the number of cells of a call, the
+ * cooperative or the persistent kernel. */
+#define GCCHEM_B200_AUTO (-1)
 #define GCCHEM_B200_PLAIN 0
 #define GCCHEM_B200_PERSISTENT 1
 #define GCCHEM_B200_PLAIN_FUSED 2
@@ -108,11 +111,29 @@ void gcchem_b200_sizes(int* nvar, int* nfix, int* nreact, int* nnz);
  * gcchem_b200_set_row_scratch; 0 = default 128);
  * blocks_per_sm: resident blocks the persistent and cooperative grids assume
  * (0 = the occupancy calculator's maximum).  Returns 0, or -1 for invalid
- * values.  Until set_launch or the environment names a kernel, every call
- * takes the cooperative or the persistent one by its number of cells.  The
- * environment
- * variables GCCHEM_B200_MODE (plain|persistent|plain_fused|coop),
- * GCCHEM_B200_THREADS and GCCHEM_B200_BLOCKS_PER_SM set the defaults. */
+ * values.  The environment variables GCCHEM_B200_MODE
+ * (auto|plain|persistent|plain_fused|coop), GCCHEM_B200_THREADS and
+ * GCCHEM_B200_BLOCKS_PER_SM set the defaults.
+ *
+ * In the automatic mode a call of up to 16,000 cells (4,000 in the
+ * --fmad=false build; any number, in the FMA build, for a mechanism without
+ * the generated factorisation) takes the cooperative kernel, with 128 threads
+ * per cell and as many blocks as fit, a larger one the persistent kernel with
+ * the given threads and blocks.
+ *
+ * One named kernel gives a cell the same bits in a call of any size.  The
+ * kernels of the FMA build differ from one another in rounding (1e-8 and more
+ * in the step sizes of a few cells in 10^5, whose steps amplify it), so in the
+ * automatic mode a cell's result depends on which side of the line its call is:
+ * on the number of ranks, devices or slices over which a grid is split.  Where
+ * that must not be, name a kernel, or use the --fmad=false build, whose kernels
+ * all give the same bits.
+ *
+ * The adjoint (gcchem_b200_adjoint_device) follows a rule of its own: one block
+ * per cell up to 16,000 cells (any number without the generated factorisation)
+ * in the automatic, persistent and cooperative modes of the FMA build, one
+ * thread per cell for more cells, in the plain modes and in the --fmad=false
+ * build. */
 int gcchem_b200_set_launch(int mode, int threads, int blocks_per_sm);
 
 /* Where the indexed factorisation (KppDecomp, used by mechanisms without the
