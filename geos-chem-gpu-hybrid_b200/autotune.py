@@ -8,7 +8,8 @@ Picks, for one device / mechanism / arithmetic variant, the fastest of:
   (resident grid draining the cost-ordered queue, generated register-blocked
   LU) or ``coop`` (one thread block per cell draining the same queue, the
   cell's factors and vectors in shared memory: the thread-per-cell versus
-  block-cooperative choice);
+  block-cooperative choice), or ``auto``, the library's own choice between
+  coop and persistent by the number of cells of each call;
 * cells (threads) per block: 64, 128 or 256 (threads per cell for coop);
 * resident blocks per SM the persistent grid assumes (occupancy maximum, or 1);
 * for the plain kernels, the workspace layout: one launch over the whole
@@ -22,7 +23,11 @@ The persistent kernel's workspace is bounded by the resident threads
 (~4.7 GB for fullchem) while a plain launch's grows with the batch, which
 the capped sample does not show (it is smaller, and its cells take no warm
 steps), so another candidate must beat the best persistent one by
-``PREFER_PERSISTENT`` to be chosen.
+``PREFER_PERSISTENT`` to be chosen.  A named kernel is the one that this batch
+wants, and every other call of the process then gets it too: a process tuned
+on a large grid would solve a 72-cell column in 0.4 s instead of 11 ms.  It
+must therefore beat the automatic choice, with any block size, by
+``PREFER_AUTO``, which is above what repeated timings of one kernel differ by.
 
 Every candidate solves the same strided sample of the caller's batch with
 the step count capped (ICNTRL(4) = ``cap``), so a candidate costs well under
@@ -43,6 +48,8 @@ import numpy as np
 # (kernel, threads per block, persistent blocks per SM, plain cells per launch,
 #  row scratch of the indexed factorisation)
 CANDIDATES = [
+    ("auto", 128, 0, 0, "global"), ("auto", 64, 0, 0, "global"),
+    ("auto", 256, 0, 0, "global"), ("auto", 128, 1, 0, "global"),
     ("coop", 128, 0, 0, "global"), ("coop", 256, 0, 0, "global"),
     ("persistent", 128, 0, 0, "global"), ("persistent", 64, 0, 0, "global"),
     ("persistent", 256, 0, 0, "global"), ("persistent", 128, 1, 0, "global"),
@@ -55,6 +62,7 @@ CANDIDATES = [
 # the large grids: layout and chunk size of the plain kernels against the
 # persistent kernel's resident-thread workspace
 CHUNKED = [
+    ("auto", 256, 0, 0, "global"), ("auto", 128, 0, 0, "global"),
     ("coop", 128, 0, 0, "global"),
     ("persistent", 256, 0, 0, "global"), ("persistent", 128, 0, 0, "global"),
     ("plain_fused", 128, 0, 32768, "global"), ("plain_fused", 128, 0, 65536, "global"),
@@ -62,6 +70,7 @@ CHUNKED = [
     ("plain", 128, 0, 131072, "global"),
 ]
 PREFER_PERSISTENT = 1.05
+PREFER_AUTO = 1.03
 
 
 def cache_path() -> str:
@@ -99,9 +108,9 @@ def _store(solver, entry, tag="default") -> None:
 
 
 def apply(solver, entry) -> None:
-    from .binding import PLAIN, PERSISTENT, PLAIN_FUSED, COOP
-    mode = {"plain": PLAIN, "plain_fused": PLAIN_FUSED, "coop": COOP}.get(entry["mode"],
-                                                                          PERSISTENT)
+    from .binding import AUTO, PLAIN, PERSISTENT, PLAIN_FUSED, COOP
+    mode = {"auto": AUTO, "plain": PLAIN, "plain_fused": PLAIN_FUSED,
+            "coop": COOP}.get(entry["mode"], PERSISTENT)
     shared = entry.get("scratch", "global") == "shared"
     if not shared:
         solver.set_row_scratch(False)
@@ -113,8 +122,11 @@ def apply(solver, entry) -> None:
 
 def _score(entry) -> float:
     """Throughput, with a bounded workspace (the persistent kernel's) or none
-    (the cooperative kernel's) worth PREFER_PERSISTENT."""
-    w = PREFER_PERSISTENT if entry["mode"] in ("persistent", "coop") else 1.0
+    (the cooperative kernel's) worth PREFER_PERSISTENT, and the automatic choice
+    between the two PREFER_AUTO more."""
+    w = PREFER_PERSISTENT if entry["mode"] in ("auto", "persistent", "coop") else 1.0
+    if entry["mode"] == "auto":
+        w *= PREFER_AUTO
     return entry["cells_per_s"] * w
 
 
