@@ -1,10 +1,11 @@
 """Gradients of a chemistry step through torch.autograd.
 
 ``ChemistryStep.apply(C0, log_rconst, solver, controls)`` solves one
-chemistry step of every cell on the GPU (forward: checkpointed persistent
-solve) and returns the final concentrations; ``backward`` runs the discrete
-adjoint kernel (csrc/adjoint.cu) through the recorded step sequence and
-returns dL/dC0 (variable species; fixed species get 0) and
+chemistry step of every cell on the GPU (forward: a solve that stores
+checkpoints) and returns the final concentrations; ``backward`` runs the discrete
+adjoint kernel (one block per cell, csrc/coop_adjoint.cuh, or one thread per
+cell, csrc/adjoint.cu, by the number of cells) through the recorded step
+sequence and returns dL/dC0 (variable species; fixed species get 0) and
 dL/d log RCONST.  Tensors use the device layout of the C-ABI: C (n, NSPEC),
 RCONST (n, NREACT), float64 on the GPU.
 

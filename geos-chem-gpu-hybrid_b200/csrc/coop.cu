@@ -10,7 +10,8 @@
  * rates are in shared memory (110 KB for fullchem), the state and the stage
  * vectors in registers, so a solve reads HBM only to load a cell and store its
  * result, and an attempt takes 72 us.  A block holds one cell, or two when
- * there are more cells than SMs.  The groups drain the same cost-ordered queue
+ * there are more cells than one-cell blocks fit on the GPU (two per SM for both
+ * shipped mechanisms: 296 cells on 148 SMs).  The groups drain the same cost-ordered queue
  * as the persistent kernel.
  *
  * Parallelism inside a cell comes from the instruction streams that
@@ -443,7 +444,7 @@ __device__ __forceinline__ double coop_chain(const double* sm, int first, int bl
    the warps, columns over the lanes.  A step scales the pivot row in its warp,
    hands it over through A (free here; two rows in turn, so that one barrier per
    step is enough) and updates the other rows, their factors coming from the
-   pivot column's lane.  ~250 cycles a step; the 62-level program that walked
+   pivot column's lane.  ~250 cycles a step; the 61-level program that walked
    these pivots took 49 of its levels, ~1,000 cycles each, for them. */
 template <int NT, int NG>
 __device__ __forceinline__ void coop_tail(double* sm) {
@@ -952,7 +953,8 @@ static size_t coop_smem_bytes(int threads, int cells) {
   return ((size_t)cells * cell + COOP_NCOEF) * sizeof(double);
 }
 
-/* cells per block of the shared form */
+/* cells per block of the shared form: fullchem's shared memory (110 KB a cell)
+   and both mechanisms' registers (228 and 254 per thread) hold no third */
 #define COOP_NG 2
 
 /* the kernel instances: threads per cell (128 or 256), cells per block */

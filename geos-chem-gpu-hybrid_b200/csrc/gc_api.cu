@@ -38,19 +38,22 @@ const int kMaxDev = 64;
 
 /* The cooperative kernel solves a cell in a thirtieth of the time one thread
    takes, but keeps only two cells per SM; one thread per cell catches up once
-   the batch fills the GPU several times.  Full cold steps on a B200,
-   cooperative / persistent: fullchem 1 cell 0.008 / 0.27 s, 1,000 cells 0.033 /
-   0.555 s, 16,000 cells 0.41 / 1.08 s, 29,952 cells 0.76 / 1.19 s; at full load
-   3.4 M / 4.6 M attempts per second.  The line is drawn below the crossover
-   (about 50,000 cells): one cell in 10^5 has a step-size sequence that
-   amplifies any difference in rounding to 1e-8 and more, so that only batches
-   that gain at least twofold leave the arithmetic of the thread-per-cell
-   kernels.  Without the fused factorisation (synthetic mechanism) the
-   cooperative kernel wins at every size: 1,500 cells 0.019 / 0.66 s, 2.6 M /
-   0.8 M attempts per second at full load.  The --fmad=false build may not
-   split sums over lanes, and its two kernels give the same bits: fullchem 100
-   cells 0.11 / 0.58 s, 1,000 cells 0.24 / 0.76 s, 4,000 cells 0.76 / 1.18 s, 8,000
-   cells 1.46 / 1.30 s; synthetic 1,500 cells 0.24 / 0.74 s. */
+   the batch fills the GPU several times.  Cold 1200 s steps of independent cells
+   (workloads.plain_small, synthetic_stiff) on a B200, cooperative / persistent:
+   fullchem 1 cell 0.006 / 0.21 s, 1,000 cells 0.032 / 0.59 s, 16,000 cells 0.40 /
+   1.04 s, 29,952 cells 0.75 / 1.17 s, 50,000 cells 1.24 / 1.66 s; at full load
+   3.4 M / 4.6 M attempts per second.  The line is therefore not where the times
+   meet, which is above 50,000 cells: it bounds the calls whose bits changed when
+   the cooperative kernel became the default.  The two kernels round the same
+   arithmetic differently, and one cell in 10^5 has a step-size sequence that
+   amplifies that to 1e-8 and more; neither is the more accurate.  A call above
+   the line gains less than a call below it (2.6-fold at 16,000 cells, 1.6-fold at
+   29,952) and keeps the thread-per-cell kernels' bits.  Without the fused
+   factorisation (synthetic mechanism) the cooperative kernel wins at every size:
+   1,500 cells 0.12 / 4.4 s, 3.3 M / 0.8 M attempts per second at full load.  The
+   --fmad=false build may not split sums over lanes, and its two kernels give the
+   same bits, so its line is where it pays: fullchem 100 cells 0.11 / 0.59 s,
+   1,000 cells 0.22 / 0.81 s, 4,000 cells 0.75 / 1.21 s, 8,000 cells 1.47 / 1.32 s. */
 #if defined(GC_LU_RECIP) && GC_LU_RECIP
 const int kCoopCells = 16000;
 const bool kCoopAlways = true;      /* without the fused factorisation */

@@ -7,8 +7,10 @@ mechanism IR into those lists, ``coop_inc`` emits them as C arrays.  The two
 forms (split or not), the levels, the inverses of the sweeps and the format of
 the words are described where they are built.
 
-``compile_tables`` holds the expressions themselves as flat tables; it decides
-whether a mechanism's expressions have a shape that the programs support.
+``compile_tables`` holds the expressions themselves as flat tables, with the
+factorisation and the solves as lists of updates in the reference's order.  The
+kernel does not read them: they refuse expressions of an unknown shape, and the
+CPU tests evaluate them as the plain form of what the programs compute.
 
 Expressions.  Every rate A(j), production P_VAR(i), destruction D_VAR(i),
 Jacobian partial B(m) and entry JVS(k) of the IR is a left-associated
@@ -102,8 +104,8 @@ def _sum_terms(node, consts):
 
 
 def compile_tables(mech: dict):
-    """All tables of the cooperative kernel, or None when some expression
-    falls outside the supported shapes."""
+    """The mechanism's plain tables (see the module's docstring), or None when
+    some expression falls outside the supported shapes."""
     n, nnz = mech["nvar"], mech["nnz"]
     nreact, nb = mech["nreact"], mech["nb"]
     crow, diag, icol = mech["lu_crow"], mech["lu_diag"], mech["lu_icol"]
@@ -210,7 +212,7 @@ def compile_tables(mech: dict):
 # The elimination order of a sparse mechanism is a chain of rows, but its
 # dependencies are shallow: in fullchem (353 species) the forward sweep has 37
 # levels, the backward sweep 33 and the factorisation, taken entry by entry,
-# 62.  Every phase of the solver is therefore a program of levels; the entries
+# 61.  Every phase of the solver is therefore a program of levels; the entries
 # of a level are independent.  An entry is computed by a group of 1, 2, 4 .. 32
 # consecutive lanes that share its products:
 #
@@ -248,7 +250,8 @@ def compile_tables(mech: dict):
 # consecutive levels form a part whose rows get the entries of the inverse of
 # their diagonal block, so that a part is solved by one level (its rows'
 # products with the inverse) after one level that subtracts the terms outside
-# the part.  fullchem: 5 parts, 8 levels instead of 70.  The inverses are rows
+# the part.  fullchem: two parts of each sweep and the tail block, 9 levels
+# instead of 69.  The inverses are rows
 # of the same recurrence as the factors and are formed by the factorisation's
 # program, next to the entries that become final at the same level:
 #
@@ -260,7 +263,7 @@ def compile_tables(mech: dict):
 # with c over the row's columns inside the part.
 #
 # The last rows are nearly dense and their pivots follow one another, two
-# levels each (fullchem: 49 of the 62 levels belong to the last 32 rows).  They
+# levels each (fullchem: 49 of the 61 levels belong to the last 32 rows).  They
 # are left out of the levels: the program only forms their Schur complement,
 # which one block-wide Gauss-Jordan elimination turns into its negative inverse,
 # rows over warps and columns over lanes; the sweeps then need one level for

@@ -121,3 +121,13 @@ def test_more_long_sums_than_lanes():
     p = coop.level_programs(m, True, 4)
     assert len(p["chains"][1]) > 32
     assert "#define COOP_CHAINS 2" in coop.coop_inc(m)
+
+
+@pytest.mark.parametrize("name,split,lu,sweep", [
+    ("fullchem", False, 61, 69), ("fullchem", True, 13, 9), ("synth120", False, 140, 143), ("synth120", True, 20, 5)])
+def test_barriers_of_a_factorisation_and_a_solve(name, split, lu, sweep):
+    """The level counts that the kernel's comments state."""
+    p = coop.level_programs(codegen.load(name), split, 4)
+    for seg, want in (("lu", lu), ("sweep", sweep)):
+        for ops in p["segs"][seg].ops:
+            assert sum(op[0][1] >> coop.L_SYNC for op in ops) == want
