@@ -298,6 +298,7 @@ NO_ENTRY = 0xFFFF      # single operations: an idle pair
 # transposed inverse]), t_j = S_j . u per reaction (tj), the partials
 # dA(j)/dV(i) of every rate (apart), and per species the sums of t_j times a
 # partial and of t_j times its derivative along a stage vector (vthl).
+ADJOINT = ("sweept", "tj", "apart", "vthl")
 
 LONG = 60              # terms of Fun's sums above which a sum goes through the buffer
 
@@ -981,7 +982,7 @@ def coop_inc(mech: dict) -> str:
             p = forms[split, nw]
             rounds = max([1] + [-(-len(c) // 32) for c in p["chains"]])
             if nw == 4:
-                lines += [f"#define COOP_NX {p['nx']}", f"#define COOP_NEXT {len(p['ext'])}",
+                lines += [f"#define COOP_NX {p['nx']}",
                           f"#define COOP_NEXTRA {len(p['extra'])}", f"#define COOP_PARTS {p['parts']}",
                           doubles("coop_ext", p["ext"]),
                           arr("int", "coop_extra_src", [j for j, _ in p["extra"]]),
@@ -998,10 +999,13 @@ def coop_inc(mech: dict) -> str:
                               [f"(q) == {k} ? {v}" for k, v in enumerate(p["nbp"])] + ["0"]),
                           arr("int", "coop_diag", [o << 1 | (e and 1) for o, e in p["diag"]])]
                 lines += [f"#define COOP_SEG_{name.upper()} {k}" for k, name in enumerate(p["segs"])]
-            lines += [arr("int", f"coop_place_t{nw}", p["place_t"]), f"#define COOP_NG{nw} {p['ng']}",
+                lines.append(arr("int", f"coop_place_t{nw}", p["place_t"]))
+            lines += [f"#define COOP_NG{nw} {p['ng']}",
                       f"#define COOP_CELL{nw} {p['cell']}", arr("int", f"coop_place{nw}", p["place"])]
             words, where = [], []
-            for seg in p["segs"].values():
+            for name, seg in p["segs"].items():
+                if nw == 8 and name in ADJOINT:      # the adjoint has 4 warps
+                    continue
                 for ops in seg.ops:
                     where.append("{%d,%d}" % (len(words) // 4, len(ops)))
                     for op in ops:                   # first four words of the lanes, then the others
