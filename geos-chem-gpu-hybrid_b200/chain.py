@@ -4,7 +4,7 @@ One chemistry step of the model's batched GPU path, done entirely on the
 device and stream-ordered, so that several steps can be captured into one
 CUDA graph and replayed:
 
-1. solve every cell (gcchem_b200_integrate_device, persistent queue);
+1. solve every cell (gcchem_b200_integrate_device, cost-ordered queue);
 2. clamp negative concentrations to zero, as the model's scatter does
    (``C(N) = MAX(C(N), 0)``, src/geos-chem/GeosCore/fullchem_mod.F90:2995);
 3. warm start: RCNTRL(3) <- RSTAT(3) (Hnew; the model keeps it in

@@ -218,7 +218,7 @@ int gcchem_b200_adjoint_device(int nCell, const double* C0, const double* RCONST
                                const double* lam, double* gC0, double* gK, int* ierr,
                                void* stream);
 
-/* Device-side cost ordering for the persistent queue: writes to `order`
+/* Device-side cost ordering for the persistent and cooperative kernels' queue: writes to `order`
  * (device, nCell ints) the columns 0..nCell-1 sorted by descending cost key
  * (device, nCell ints, any int32 value), cells with equal keys in increasing
  * column order.  With the previous chemistry step's ISTAT(3) as keys this is
